@@ -71,7 +71,7 @@ def listed():
         dict(name="strip3d_f64_exact", kind="strip3d", nx=97, ny=114, nz=187, P=10, gap=10, port_gap=20, steps=1200,
              nf=21, source="TM", prec="f64", arith="exact"),
         # the largest: the large run's cross-section, 38 M cells
-        dict(name="rib3d_f32", kind="rib3d", nx=384, ny=384, nz=256, steps=1000, nf=41, prec="f32", arith="fast"),
+        dict(name="rib3d_f32", kind="rib3d", nx=384, ny=384, nz=256, steps=1000, nf=5, prec="f32", arith="fast"),
         # a scattering-loss realization
         dict(name="scatter_f32", kind="scatter", length_um=5.0, ppw=20, flights=1.2, source="TM", prec="f32",
              arith="fast"),
@@ -117,7 +117,7 @@ def draw(rng):
                     flights=round(rng.uniform(1.0, 1.3), 2), source=rng.choice(["TE", "TM"]), prec="f32", arith="fast")
     if kind == "rib3d":
         return dict(kind=kind, nx=rng.randint(200, 380), ny=rng.randint(200, 380), nz=rng.randint(180, 256),
-                    steps=rng.randint(800, 1000), nf=21, prec="f32", arith="fast")
+                    steps=rng.randint(800, 1000), nf=5, prec="f32", arith="fast")
     if kind == "batch":
         return dict(kind=kind, count=rng.randint(2, 4), steps=rng.randint(1000, 1500), nf=rng.choice([21, 41]),
                     draw=rng.randint(1, 10 ** 6))
