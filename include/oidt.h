@@ -114,7 +114,8 @@ typedef struct oidt_job_desc {
    *              4 = tile form: each block advances a tile of the grid and a
    *                  halo around it through sub-blocks of up to 8 steps in
    *                  shared memory; a ring block is one cooperative launch
-   *                  where every tile is resident at once;
+   *                  where every tile is resident at once, and so is a
+ *                  block of up to 128 steps of a long advance;
    * reserved[1]: 1 = launch every step directly (no CUDA-graph replay);
    * reserved[2]: 3D per-cell form: rows of a block's 32 x rows tile,
    *              2, 4 or 8 (0 = 4); 2D tile form: 1 = one launch per

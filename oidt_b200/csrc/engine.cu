@@ -43,6 +43,7 @@
 #include "sweep3d.cuh"
 #include "vec3d.cuh"
 #include "tile2d.cuh"
+#include "strip2d.cuh"
 
 using namespace oidt;
 
@@ -56,7 +57,9 @@ constexpr int TY = kSweepTY, TZ = kSweepTZ, ST = kSweepStages;  // owned tile of
 constexpr int EYB = kSweepEY, EZB = kSweepEZ;                      // its thread box
 constexpr int kVariantCell = 0, kVariantSweep = 1, kVariantVec = 2, kVariantWave = 3;  // oidt_job_desc.reserved[0]
 constexpr int kVariantTile = 4;  // 2D: tiles advanced in sub-blocks of up to kTileHaloMax steps (tile2d.cuh)
+constexpr int kTileLongBlock = 128;  // steps of a 2D tile-form job's long block at most (a multiple of its ring block)
 constexpr int kTileMaxBlocks = 1024;  // tiles of a cooperative (several sub-block) launch at most
+constexpr long long kStripCoopCells = 148LL * kStripThreads * kStripCells;  // cells of a grid one cooperative strip launch holds at most
 constexpr size_t kTileSmemMax = 227 * 1024;  // shared memory of a tile block at most
 
 // ---------------------------------------------------------------------------
@@ -366,10 +369,12 @@ struct JobPlan {
   size_t off_mat, off_mtab;       // material index [nx][ny][nzp] and table [256][4] (3D, optional)
   bool mat;
   size_t off_wave;                // ordered form: E-block counts per plane (after 8 spare bytes)
-  size_t off_tile;                // 2D tile form: sub-blocks completed per tile [kTileMaxBlocks]
+  size_t off_tile;                // 2D tile form: sub-blocks completed per tile [kTileMaxBlocks] ...
+  bool strip;                     // ... the strip kernel (float32 fast; else one cell a thread) ...
+  size_t off_xch, xch_words;      // ... and its exchange words (0: none)
   size_t off_pow;                 // port power [nf] complex float64
   long long N, plane;
-  int K, esz, nzp, nbuf, variant, L, nitems;
+  int K, KL, esz, nzp, nbuf, variant, L, nitems;  // K: steps of a ring block; KL: of a long block (K but for the tile form)
   int rows;  // 3D per-cell tile rows
   int psi_pitch;  // row length along z of the 3D x- and y-slab psi arrays (nz or nzp)
   int psz;        // row length of the 3D z-slab psi arrays (P, or the vector form's padded rows) ...
@@ -582,7 +587,11 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
             L.take(psi_elems(d->mode, fa.second, d->nx, d->ny, d->nz, P, psi_pitch, zr.pitch) * esz);
   pl->off_jsrc = L.take((size_t)d->nt * esz);
   for (int t = 0; t < 4; ++t) pl->off_tw[t] = L.take((size_t)d->nf * d->nt * 8);
-  pl->off_ring = L.take((size_t)K * 2 * nslot_of(d->mode) * plane * esz);
+  // Tile form: a ring of KL >= K steps.  An advance of KL steps or more replays blocks of KL, whose launch, set-up
+  // and fold (7 us a block, a fifth of a 32-step block of a 400 x 200 slab) are paid once; multi-job blocks stay K.
+  // Planes of 20000 cells and more keep blocks of K: their steps are far longer, their rings not small.
+  const int KL = variant == kVariantTile && K < kTileLongBlock && plane < 20000 ? kTileLongBlock / K * K : K;
+  pl->off_ring = L.take((size_t)KL * 2 * nslot_of(d->mode) * plane * esz);
   pl->off_acc = L.take((size_t)2 * ncomp_of(d->mode) * d->nf * plane * 16);
   pl->off_state = L.take(64);
   pl->off_pow = L.take((size_t)d->nf * 16);
@@ -592,7 +601,14 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
     pl->off_mtab = L.take((size_t)256 * 4 * esz);
   }
   if (variant == kVariantWave) pl->off_wave = L.take(8 + (size_t)4 * (d->ie - d->ib));
-  if (variant == kVariantTile) pl->off_tile = L.take((size_t)4 * kTileMaxBlocks);
+  if (variant == kVariantTile) {
+    pl->off_tile = L.take((size_t)4 * kTileMaxBlocks);
+    // the strip kernel's exchange words (34 MB at most), for grids a cooperative launch can hold
+    pl->strip = d->precision == OIDT_F32 && d->arith == OIDT_ARITH_FAST;
+    pl->xch_words = pl->strip && d->reserved[2] == 0 && N <= kStripCoopCells && (long long)P * (d->nx + d->ny) <= kStripCoopCells
+                        ? 2 * strip2d_xch_buf(d->nx, d->ny, P) : 0;
+    pl->off_xch = L.take(8 * pl->xch_words);
+  }
   if (d->probe[0] == 1) {
     pl->probe_bytes = (size_t)4 * d->nt * d->nx * esz;
     pl->off_probe = L.take(pl->probe_bytes);
@@ -608,6 +624,7 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
   pl->N = N;
   pl->plane = plane;
   pl->K = K;
+  pl->KL = KL;
   pl->rows = rows;
   pl->psi_pitch = psi_pitch;
   pl->psz = zr.pitch;
@@ -631,8 +648,8 @@ struct Job {
   FoldParams<float> ff{};
   FoldParams<double> fd{};
   int parity = 0;                                 // buffer holding the current state
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};  // K-step block starting at parity 0 / 1
-  long long graph_launches = 0;                   // kernels per graph replay
+  cudaGraphExec_t graph[4] = {};                  // K-step block starting at parity 0 / 1, KL-step block the same
+  long long graph_launches[4] = {};               // kernels per graph replay
   cudaEvent_t ready = nullptr;                    // uploads finished
   cudaEvent_t done = nullptr;                     // last enqueued work finished
   long long steps_enqueued = 0;
@@ -642,6 +659,7 @@ struct Job {
   int tile_blocks = 0;                  // ... blocks (tiles) of a launch
   bool tile_coop = false;               // ... a ring block is one cooperative launch of sub-blocks
   size_t tile_smem = 0;                 // ... shared memory of a block
+  StripArgs strip{};                    // ... the strip kernel's split (in place of `tile`)
 };
 
 constexpr int kAuxStreams = 64;  // a served request is two jobs; the mix keeps ~40 active
@@ -780,7 +798,7 @@ template <typename T> void fill_params(Job *J) {
     if (d.mode != OIDT_MODE_YEE3D) { p.slo[2] = 0; p.shi[2] = 1; }
     p.jsrc = reinterpret_cast<const T *>(m + pl.off_jsrc);
     p.ring = reinterpret_cast<T *>(m + pl.off_ring);
-    p.ring_K = pl.K;
+    p.ring_K = pl.KL;
     p.nslot = nslot_of(d.mode);
     p.plane = pl.plane;
     p.port_pos[0] = d.port_pos[0];
@@ -976,23 +994,16 @@ template <typename T, bool EXACT> void v3_wave(Job *J, bool pdl, const Params<T>
   else k_v3_wave<T, EXACT><<<grd, blk, 0, st>>>(p, g, w, s);
 }
 
-// One launch of the 2D tile form (k_2d_tile): steps s0 .. s0 + cnt - 1 of a
-// ring block, read from buffer p.f / p.psi, owned cells written to p.fn /
-// p.psin.
-// cnt > halo: one cooperative launch of ceil(cnt / halo) sub-blocks.
-template <typename T, bool EXACT>
-void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStream_t st) {
-  void (*kern)(Params<T>, TileArgs) =
-      p.mode == OIDT_MODE_TM2 ? k_2d_tile<T, EXACT, OIDT_MODE_TM2> : k_2d_tile<T, EXACT, OIDT_MODE_TE2>;
-  TileArgs a = J->tile;
-  a.s0 = s0;
-  a.cnt = cnt;
-  a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
-  if (cnt > a.halo) {
+// A launch of the tile form's kernel: cooperative (several sub-blocks), or
+// with or without programmatic serialization.
+template <typename K, typename PT, typename AT>
+void tile_launch_as(K kern, bool coop, bool pdl, int blocks, int threads, size_t smem, cudaStream_t st, const PT &p,
+                    const AT &a) {
+  if (coop) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(J->tile_blocks);
-    cfg.blockDim = dim3(kTileThreads);
-    cfg.dynamicSmemBytes = J->tile_smem;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1001,14 +1012,48 @@ void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStre
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kern, p, a);
   } else if (pdl) {
-    launch_step_kernel(kern, dim3(J->tile_blocks), dim3(kTileThreads), J->tile_smem, st, p, a);
+    launch_step_kernel(kern, dim3(blocks), dim3(threads), smem, st, p, a);
   } else {
-    kern<<<J->tile_blocks, kTileThreads, J->tile_smem, st>>>(p, a);
+    kern<<<blocks, threads, smem, st>>>(p, a);
   }
 }
 
-// Launches of the 2D tile form for cnt steps: up to halo steps each.
-int tile_launches(const Job *J, int cnt) { return (cnt + J->tile.halo - 1) / J->tile.halo; }
+template <int MODE> void (*strip_kernel(int cells))(const Params<float>, StripArgs) {
+  return cells == 1 ? k_2d_strip<MODE, 1> : k_2d_strip<MODE, 4>;
+}
+
+// One launch of the 2D tile form (k_2d_strip in float32 fast arithmetic, else
+// k_2d_tile): steps s0 .. s0 + cnt - 1 of a ring block, read from buffer
+// p.f / p.psi, owned cells written to p.fn / p.psin.  cnt > halo: one
+// cooperative launch of ceil(cnt / halo) sub-blocks.
+template <typename T, bool EXACT>
+void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStream_t st) {
+  if constexpr (sizeof(T) == 4 && !EXACT) {
+    StripArgs a = J->strip;
+    a.s0 = s0;
+    a.cnt = cnt;
+    a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
+    a.xch = reinterpret_cast<unsigned long long *>(J->mem + J->pl.off_xch);
+    a.xbuf = (long long)J->pl.xch_words / 2;
+    tile_launch_as(p.mode == OIDT_MODE_TM2 ? strip_kernel<OIDT_MODE_TM2>(a.cells) : strip_kernel<OIDT_MODE_TE2>(a.cells),
+                   cnt > a.halo, pdl, J->tile_blocks, a.threads, J->tile_smem, st, p, a);
+    return;
+  }
+  void (*kern)(Params<T>, TileArgs) =
+      p.mode == OIDT_MODE_TM2 ? k_2d_tile<T, EXACT, OIDT_MODE_TM2> : k_2d_tile<T, EXACT, OIDT_MODE_TE2>;
+  TileArgs a = J->tile;
+  a.s0 = s0;
+  a.cnt = cnt;
+  a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
+  tile_launch_as(kern, cnt > a.halo, pdl, J->tile_blocks, kTileThreads, J->tile_smem, st, p, a);
+}
+
+// Launches of the 2D tile form for cnt steps: up to halo steps each -- also the
+// buffer flips of k_2d_tile's cooperative launch; k_2d_strip's is one flip.
+int tile_halo(const Job *J) { return J->pl.strip ? J->strip.halo : J->tile.halo; }
+int tile_launches(const Job *J, int cnt) {
+  return J->pl.strip && J->tile_coop ? 1 : (cnt + tile_halo(J) - 1) / tile_halo(J);
+}
 
 template <typename T> size_t sweep_smem() { return sweep_smem_bytes<T, EYB, EZB, ST>(); }
 
@@ -1105,8 +1150,8 @@ template <typename T, bool EXACT> void launch_steps(oidt_ctx *ctx, Job *J, int c
     }
     const int nl = tile_launches(J, cnt);
     for (int l = 0; l < nl; ++l) {
-      const int s0 = l * J->tile.halo;
-      tile_launch<T, EXACT>(true, J, views<T>(J)[par ^ (l & 1)], s0, std::min(J->tile.halo, cnt - s0), st);
+      const int s0 = l * tile_halo(J);
+      tile_launch<T, EXACT>(true, J, views<T>(J)[par ^ (l & 1)], s0, std::min(tile_halo(J), cnt - s0), st);
     }
     ctx->launches += nl;
     return;
@@ -1118,19 +1163,20 @@ template <typename T, bool EXACT> void launch_steps(oidt_ctx *ctx, Job *J, int c
 // The job's K-step block starting on buffer parity par (its steps, then its
 // DFT fold) as a CUDA graph, captured on stream st at first use.  Capture
 // enqueues nothing, so st may hold work of other jobs.
-template <typename T, bool EXACT> int job_graph(oidt_ctx *ctx, Job *J, int par, cudaStream_t st) {
-  if (J->graph[par]) return OIDT_OK;
-  const int K = J->pl.K;
+// lng: the job's long block (KL steps) instead.
+template <typename T, bool EXACT> int job_graph(oidt_ctx *ctx, Job *J, int par, cudaStream_t st, bool lng = false) {
+  const int k = lng ? 2 + par : par, K = lng ? J->pl.KL : J->pl.K;
+  if (J->graph[k]) return OIDT_OK;
   cudaGraph_t g;
   const long long before = ctx->launches;
   CU(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
   launch_steps<T, EXACT>(ctx, J, K, par, st);
   launch_fold<T, EXACT>(ctx, J, K, st);
   CU(ctx, cudaStreamEndCapture(st, &g));
-  const cudaError_t ie = cudaGraphInstantiate(&J->graph[par], g, 0);
+  const cudaError_t ie = cudaGraphInstantiate(&J->graph[k], g, 0);
   cudaGraphDestroy(g);
   CU(ctx, ie);
-  J->graph_launches = ctx->launches - before;
+  J->graph_launches[k] = ctx->launches - before;
   ctx->launches = before;
   return OIDT_OK;
 }
@@ -1141,13 +1187,15 @@ template <typename T, bool EXACT> int advance_t(oidt_ctx *ctx, Job *J, int nstep
   const int K = J->pl.K;
   int left = nsteps;
   while (left > 0) {
-    const int cnt = std::min(K, left);
+    const bool lng = left >= J->pl.KL && J->pl.KL > K;
+    const int cnt = lng ? J->pl.KL : std::min(K, left);
     const int par = J->parity;
-    if (cnt == K && J->d.reserved[1] == 0) {
-      int rc = job_graph<T, EXACT>(ctx, J, par, st);
+    if (cnt >= K && J->d.reserved[1] == 0) {
+      int rc = job_graph<T, EXACT>(ctx, J, par, st, lng);
       if (rc) return rc;
-      CU(ctx, cudaGraphLaunch(J->graph[par], st));
-      ctx->launches += J->graph_launches;
+      const int k = lng ? 2 + par : par;
+      CU(ctx, cudaGraphLaunch(J->graph[k], st));
+      ctx->launches += J->graph_launches[k];
     } else {
       launch_steps<T, EXACT>(ctx, J, cnt, par, st);
       launch_fold<T, EXACT>(ctx, J, cnt, st);
@@ -1192,7 +1240,7 @@ template <typename T, bool EXACT> int batch_block(oidt_ctx *ctx, std::vector<Job
     cudaStream_t sb = ctx->aux[b % na];
     if (full && J->d.reserved[1] == 0) {
       CU(ctx, cudaGraphLaunch(J->graph[J->parity], sb));
-      ctx->launches += J->graph_launches;
+      ctx->launches += J->graph_launches[J->parity];
     } else {
       launch_steps<T, EXACT>(ctx, J, cnt, J->parity, sb);
       launch_fold<T, EXACT>(ctx, J, cnt, sb);
@@ -1260,8 +1308,8 @@ template <typename T, bool EXACT> int profile_t(oidt_ctx *ctx, Job *J, int nstep
       tile_launch<T, EXACT>(false, J, views<T>(J)[J->parity], 0, nsteps, st);
     } else {
       for (int l = 0; l < nl; ++l) {
-        const int s0 = l * J->tile.halo;
-        tile_launch<T, EXACT>(false, J, views<T>(J)[J->parity ^ (l & 1)], s0, std::min(J->tile.halo, nsteps - s0), st);
+        const int s0 = l * tile_halo(J);
+        tile_launch<T, EXACT>(false, J, views<T>(J)[J->parity ^ (l & 1)], s0, std::min(tile_halo(J), nsteps - s0), st);
       }
     }
     cudaEventRecord(ev[1], st);
@@ -1356,8 +1404,8 @@ template <typename T, bool EXACT> int profile_t(oidt_ctx *ctx, Job *J, int nstep
 }
 
 void destroy_job(oidt_ctx *ctx, Job *J) {
-  for (int b = 0; b < 2; ++b)
-    if (J->graph[b]) cudaGraphExecDestroy(J->graph[b]);
+  for (cudaGraphExec_t g : J->graph)
+    if (g) cudaGraphExecDestroy(g);
   cudaFreeAsync(J->mem, ctx->stream);  // stream-ordered: no device-wide synchronisation
   cudaEventDestroy(J->ready);
   cudaEventDestroy(J->done);
@@ -1392,6 +1440,10 @@ void set_tile_attrs() {
   tile_attrs_of<float, true, OIDT_MODE_TE2>();
   tile_attrs_of<double, false, OIDT_MODE_TE2>();
   tile_attrs_of<double, true, OIDT_MODE_TE2>();
+  for (int c = 1; c <= kStripCells; c *= 4) {
+    cudaFuncSetAttribute(strip_kernel<OIDT_MODE_TM2>(c), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
+    cudaFuncSetAttribute(strip_kernel<OIDT_MODE_TE2>(c), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmemMax);
+  }
 }
 
 // The tile form's split of a job.  A held tile has at most kTileThreads
@@ -1445,6 +1497,79 @@ void tile_plan(Job *J, int sms) {
       J->tile_blocks = bb;
     }
   }
+}
+
+// The strip kernel's split of a job: strip length (1 or 4 cells), steps per
+// sub-block (the halo: 1, 2, 3, 4, 6 or 8 and at most the ring steps, or the
+// descriptor's reserved[3]), tile extents, by the least estimated cycles per
+// step.  One wave of cooperative tiles where the grid fits it with a halo no
+// wider than a tile (the halos cross through the exchange words), otherwise a
+// launch per sub-block in waves.  The estimates' constants are fits to steps
+// measured on a B200 (us per step, best of each kind: one cell a thread / four
+// / waves): 300 x 150 0.94 / 1.30 / 1.9, 400 x 200 1.13 / 1.38 / 2.2,
+// 480 x 250 2.44 / 1.48 / 2.8, 613 x 227 - / 1.57 / 2.2, 675 x 141 TE 1.55 /
+// 1.44 / 1.9, 800 x 300 - / 2.23 / 3.5, 603 x 1601 - / - / 10.9.  Among equal
+// estimates the tile nearest a square wins: 613 x 227 at 4 steps 1.60 with
+// 26 x 38 tiles, 1.71 with 13 x 76, 1.98 with 103 x 10.
+void strip_plan(Job *J, int sms, bool coop_ok) {
+  const oidt_job_desc &d = J->d;
+  const int nx = d.nx, ny = d.ny;
+  const int hmax = std::min(kStripHaloMax, J->pl.K);
+  const int h0 = d.reserved[3] > 0 ? std::min(d.reserved[3], hmax) : 1;
+  const int h1 = d.reserved[3] > 0 ? h0 : hmax;
+  double best = 1e300;
+  auto consider = [&](int C, int h, int ti, int tj, bool coop) {
+    const int gi = (nx + ti - 1) / ti, gj = (ny + tj - 1) / tj;
+    const long long tiles = (long long)gi * gj;
+    const int hi = std::min(nx, ti + 2 * h), hj = std::min(ny, tj + 2 * h);
+    const int thr = (int)align_up((size_t)((hi + C - 1) / C) * hj, 32), most = C == 1 ? 2 * kStripThreads : kStripThreads;
+    const size_t smem = strip2d_smem(hi, hj, C, J->pl.KL);
+    if (thr > most || smem > kTileSmemMax || tiles > 0x7fffffff) return;
+    const double warps = thr / 32.0, held = thr * C / 2048.0;
+    double t;
+    if (coop) {
+      if (tiles > std::min(sms, kTileMaxBlocks) || h > std::min(ti, tj)) return;
+      t = (C == 1 ? 1300.0 + 10.0 * warps + 2150.0 / h : 1850.0 + 31.0 * warps + 1900.0 / h) + 10.0 * (ti + tj);
+    } else {  // a tile's loads, set-up and stores outweigh its steps; blocks beside one another on an SM share it
+      const int res = std::max(1, std::min(most / thr, (int)(kTileSmemMax / smem)));
+      const double fill = (double)tiles / ((double)sms * res), full = res * held;
+      t = C == 1 ? (7400.0 + std::ceil(fill) * (6900.0 - 135.0 * h + full * (1750.0 * h - 1840.0))) / h
+                 : (11200.0 + (0.65 * std::ceil(fill) + 0.35 * fill) * (10000.0 + 490.0 * h + full * (930.0 + 510.0 * h))) / h;
+      if (hj % 32) t *= 1.03;  // warps that cross rows: 603 x 1601 at 6 steps 10.9 in rows of 64 held cells, 11.3 of 51
+    }
+    if (t >= best) return;
+    best = t;
+    J->strip = StripArgs{};
+    J->strip.ti = ti;
+    J->strip.tj = tj;
+    J->strip.gj = gj;
+    J->strip.halo = h;
+    J->strip.cells = C;
+    J->strip.threads = thr;
+    J->tile_blocks = (int)tiles;
+    J->tile_smem = smem;
+    J->tile_coop = coop;
+  };
+  for (int C = 1; C <= kStripCells; C *= 4)
+    for (int h = h0; h <= h1; ++h) {
+      if (h0 != h1 && h > 3 && h % 2) continue;
+      if (coop_ok && J->pl.K > h)
+        for (int gi = 1; gi <= std::min(nx, sms); ++gi) {  // as many tiles as there are SMs
+          const int ti = (nx + gi - 1) / gi, gj = std::min(ny, sms / ((nx + ti - 1) / ti));
+          consider(C, h, ti, (ny + gj - 1) / gj, true);
+        }
+      for (int nt = kStripThreads / 2; nt <= (C == 1 ? 2 : 1) * kStripThreads; nt += kStripThreads / 4)
+        for (int ti = std::min(nx, nt * C); ti > 0;) {  // rows; columns: the most nt threads hold, evened out
+          const int gi = (nx + ti - 1) / ti, st = (std::min(nx, ti + 2 * h) + C - 1) / C;
+          ti = (nx + gi - 1) / gi;
+          const int most = st > nt ? 0 : (long long)ny * st <= nt ? ny : std::min(ny, nt / st - 2 * h);
+          if (most >= 1) {
+            const int gj = (ny + most - 1) / most;
+            consider(C, h, ti, (ny + gj - 1) / gj, false);
+          }
+          --ti;
+        }
+    }
 }
 
 }  // namespace
@@ -1578,12 +1703,20 @@ int32_t oidt_job_create(oidt_ctx *ctx, const oidt_job_desc *desc, uint64_t *job)
   J->d = *desc;
   J->pl = pl;
   if (pl.variant == kVariantTile) {
-    tile_plan(J, ctx->sms);
-    J->tile_smem = tile2d_smem(pl.esz, desc->num_cpml, J->tile.ti + 2 * J->tile.halo, J->tile.tj + 2 * J->tile.halo);
-    // a ring block in one launch where every tile is resident at once and a tile's
-    // halo reaches its 8 neighbours only
-    J->tile_coop = ctx->coop && desc->reserved[2] == 0 && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
-                   J->tile.halo <= std::min(J->tile.ti, J->tile.tj) && J->pl.K > J->tile.halo;
+    if (pl.strip) {
+      strip_plan(J, ctx->sms, ctx->coop && pl.xch_words > 0);
+    } else {
+      tile_plan(J, ctx->sms);
+      J->tile_smem = tile2d_smem(pl.esz, desc->num_cpml, J->tile.ti + 2 * J->tile.halo, J->tile.tj + 2 * J->tile.halo);
+      // a ring block in one launch where every tile is resident at once and a tile's
+      // halo reaches its 8 neighbours only
+      J->tile_coop = ctx->coop && desc->reserved[2] == 0 && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
+                     J->tile.halo <= std::min(J->tile.ti, J->tile.tj) && J->pl.K > J->tile.halo;
+    }
+    if (J->tile_blocks == 0) {
+      delete J;
+      return fail(ctx, OIDT_ERR_INVALID, "tile form: no tiling of this grid");
+    }
   }
   if (cudaMallocAsync(reinterpret_cast<void **>(&J->mem), pl.total, ctx->upload) != cudaSuccess) {
     delete J;
@@ -1949,7 +2082,7 @@ int32_t oidt_job_write_field(oidt_ctx *ctx, uint64_t job, int32_t field, const v
     rc = copy_grid_h2d(ctx, J, J->mem + J->pl.off_f[b][field], src, ctx->upload);
     if (rc) return rc;
   }
-  const long long n = (long long)J->pl.K * 2 * nslot_of(J->d.mode) * J->pl.plane;
+  const long long n = (long long)J->pl.KL * 2 * nslot_of(J->d.mode) * J->pl.plane;
   const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 8);
   if (J->d.precision == OIDT_F64)
     k_ring_fill<double><<<blocks, 256, 0, ctx->upload>>>(cells<double>(J)[J->parity]);
@@ -2029,6 +2162,8 @@ int32_t oidt_job_reset(oidt_ctx *ctx, uint64_t job) {
     CU(ctx, cudaMemsetAsync(J->mem + pl.off_wave, 0, 8 + (size_t)4 * (J->d.ie - J->d.ib), st));
   if (pl.variant == kVariantTile)  // the tiles' sub-block counters: equal (zero) again
     CU(ctx, cudaMemsetAsync(J->mem + pl.off_tile, 0, (size_t)4 * kTileMaxBlocks, st));
+  if (pl.xch_words)  // ... and the exchange words with them
+    CU(ctx, cudaMemsetAsync(J->mem + pl.off_xch, 0, 8 * pl.xch_words, st));
   CU(ctx, cudaEventRecord(J->done, st));
   J->busy = true;
   J->steps_enqueued = 0;
@@ -2047,10 +2182,10 @@ int32_t oidt_job_set_wait_limit(oidt_ctx *ctx, uint64_t job, int64_t cycles) {
   for (int b = 0; b < 2; ++b) {
     J->pvf[b].wait_cycles = J->pcf[b].wait_cycles = J->wait_cycles;
     J->pvd[b].wait_cycles = J->pcd[b].wait_cycles = J->wait_cycles;
-    if (J->graph[b]) {  // captured with the old parameters: capture again at next use
-      cudaGraphExecDestroy(J->graph[b]);
-      J->graph[b] = nullptr;
-    }
+  }
+  for (cudaGraphExec_t &g : J->graph) {  // captured with the old parameters: capture again at next use
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
   }
   return OIDT_OK;
 }

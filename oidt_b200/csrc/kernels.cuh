@@ -50,12 +50,28 @@ template <> struct Ar<float, true> {
     const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
     return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
   }
+  // composite operations of an update, as the reference evaluates them
+  static __device__ __forceinline__ float curl(float e, float c, float a, float ka, float ra, float b, float kb, float rb) {
+    return add(e, mul(c, sub(div(a, ka, ra), div(b, kb, rb))));
+  }
+  static __device__ __forceinline__ float step(float e, float c, float d, float k, float r) { return add(e, div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ float psi(float b, float q, float c, float d, float k, float r) { return add(mul(b, q), div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ float inc(float e, float c, float q) { return add(e, mul(c, q)); }
+  static __device__ __forceinline__ float dec(float e, float c, float q) { return sub(e, mul(c, q)); }
 };
 template <> struct Ar<float, false> {
   static __device__ __forceinline__ float add(float a, float b) { return a + b; }
   static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
   static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
   static __device__ __forceinline__ float div(float a, float, float rb) { return a * rb; }
+  // composite operations of an update with their fusing spelled out, so that every launch form rounds alike
+  static __device__ __forceinline__ float curl(float e, float c, float a, float, float ra, float b, float, float rb) {
+    return __fmaf_rn(c, __fmaf_rn(a, ra, -__fmul_rn(b, rb)), e);
+  }
+  static __device__ __forceinline__ float step(float e, float c, float d, float, float r) { return __fmaf_rn(__fmul_rn(c, d), r, e); }
+  static __device__ __forceinline__ float psi(float b, float q, float c, float d, float, float r) { return __fmaf_rn(b, q, __fmul_rn(__fmul_rn(c, d), r)); }
+  static __device__ __forceinline__ float inc(float e, float c, float q) { return __fmaf_rn(c, q, e); }
+  static __device__ __forceinline__ float dec(float e, float c, float q) { return __fmaf_rn(-c, q, e); }
 };
 template <> struct Ar<double, true> {
   static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
@@ -70,12 +86,28 @@ template <> struct Ar<double, true> {
     const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
     return __fma_rn(__fma_rn(-b, q1, a), y, q1);
   }
+  // composite operations of an update, as the reference evaluates them
+  static __device__ __forceinline__ double curl(double e, double c, double a, double ka, double ra, double b, double kb, double rb) {
+    return add(e, mul(c, sub(div(a, ka, ra), div(b, kb, rb))));
+  }
+  static __device__ __forceinline__ double step(double e, double c, double d, double k, double r) { return add(e, div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ double psi(double b, double q, double c, double d, double k, double r) { return add(mul(b, q), div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ double inc(double e, double c, double q) { return add(e, mul(c, q)); }
+  static __device__ __forceinline__ double dec(double e, double c, double q) { return sub(e, mul(c, q)); }
 };
 template <> struct Ar<double, false> {
   static __device__ __forceinline__ double add(double a, double b) { return a + b; }
   static __device__ __forceinline__ double sub(double a, double b) { return a - b; }
   static __device__ __forceinline__ double mul(double a, double b) { return a * b; }
   static __device__ __forceinline__ double div(double a, double, double rb) { return a * rb; }
+  // composite operations of an update with their fusing spelled out, so that every launch form rounds alike
+  static __device__ __forceinline__ double curl(double e, double c, double a, double, double ra, double b, double, double rb) {
+    return __fma_rn(c, __fma_rn(a, ra, -__dmul_rn(b, rb)), e);
+  }
+  static __device__ __forceinline__ double step(double e, double c, double d, double, double r) { return __fma_rn(__dmul_rn(c, d), r, e); }
+  static __device__ __forceinline__ double psi(double b, double q, double c, double d, double, double r) { return __fma_rn(b, q, __dmul_rn(__dmul_rn(c, d), r)); }
+  static __device__ __forceinline__ double inc(double e, double c, double q) { return __fma_rn(c, q, e); }
+  static __device__ __forceinline__ double dec(double e, double c, double q) { return __fma_rn(-c, q, e); }
 };
 
 // ---------------------------------------------------------------------------
@@ -616,20 +648,19 @@ __device__ __forceinline__ void tm2_e_cell(const Params<T> &p, int i, int j, int
     const T cb = p.cb[2][c];
     const T dhy = A::sub(Hy[c + ny], Hy[c]);
     const T dhx = A::sub(Hx[c + 1], Hx[c]);
-    T e = A::add(p.f[EZ][c], A::mul(cb, A::sub(A::div(dhy, p.kd[0][i], p.rkd[0][i]),
-                                                A::div(dhx, p.kd[1][j], p.rkd[1][j]))));
+    T e = A::curl(p.f[EZ][c], cb, dhy, p.kd[0][i], p.rkd[0][i], dhx, p.kd[1][j], p.rkd[1][j]);
     if (in_src(p, EZ, i, j, 0)) e = A::sub(e, p.jsrc[n]);  // update_source :71-76
     if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {    // update_pml_ez_xinc :80-88
       T *ps = p.psi[EZ][AX][side] + (long long)d * ny + j;
-      T v = A::add(A::mul(p.be[q], *ps), A::div(A::mul(p.ce[q], dhy), p.dx, p.rdx));
+      T v = A::psi(p.be[q], *ps, p.ce[q], dhy, p.dx, p.rdx);
       *ps = v;
-      e = A::add(e, A::mul(cb, v));
+      e = A::inc(e, cb, v);
     }
     if ((q = e_slab(j, p.jb, p.je, P, d, side)) >= 0) {    // update_pml_ez_yinc :92-100
       T *ps = p.psi[EZ][AY][side] + (long long)i * P + d;
-      T v = A::add(A::mul(p.be[q], *ps), A::div(A::mul(p.ce[q], dhx), p.dx, p.rdx));
+      T v = A::psi(p.be[q], *ps, p.ce[q], dhx, p.dx, p.rdx);
       *ps = v;
-      e = A::sub(e, A::mul(cb, v));
+      e = A::dec(e, cb, v);
     }
     p.f[EZ][c] = e;
     if (i == p.port_pos[0]) capture(p, s, 0, 0, j, e);
@@ -647,23 +678,23 @@ __device__ __forceinline__ void tm2_h_cell(const Params<T> &p, int i, int j, int
   int d, side, q;
   if (i >= p.ib && i < p.ie && j > p.jb && j < p.je) {  // update_hx :53-58
     const T dez = A::sub(Ez[c - 1], Ez[c]);
-    T h = A::add(p.f[HX][c], A::div(A::mul(db, dez), p.kd[4][j], p.rkd[4][j]));
+    T h = A::step(p.f[HX][c], db, dez, p.kd[4][j], p.rkd[4][j]);
     if ((q = h_slab(j, p.jb, p.je, P, d, side)) >= 0) {   // update_pml_hx_yinc :104-112
       T *ps = p.psi[HX][AY][side] + (long long)i * P + d;
-      T v = A::add(A::mul(p.bh[q], *ps), A::div(A::mul(p.ch[q], A::sub(Ez[c], Ez[c - 1])), p.dx, p.rdx));
+      T v = A::psi(p.bh[q], *ps, p.ch[q], A::sub(Ez[c], Ez[c - 1]), p.dx, p.rdx);
       *ps = v;
-      h = A::sub(h, A::mul(db, v));
+      h = A::dec(h, db, v);
     }
     p.f[HX][c] = h;
   }
   if (i > p.ib && i < p.ie && j >= p.jb && j < p.je) {  // update_hy :62-67
     const T dez = A::sub(Ez[c], Ez[c - ny]);
-    T h = A::add(p.f[HY][c], A::div(A::mul(db, dez), p.kd[3][i], p.rkd[3][i]));
+    T h = A::step(p.f[HY][c], db, dez, p.kd[3][i], p.rkd[3][i]);
     if ((q = h_slab(i, p.ib, p.ie, P, d, side)) >= 0) {   // update_pml_hy_xinc :116-124
       T *ps = p.psi[HY][AX][side] + (long long)d * ny + j;
-      T v = A::add(A::mul(p.bh[q], *ps), A::div(A::mul(p.ch[q], dez), p.dx, p.rdx));
+      T v = A::psi(p.bh[q], *ps, p.ch[q], dez, p.dx, p.rdx);
       *ps = v;
-      h = A::add(h, A::mul(db, v));
+      h = A::inc(h, db, v);
     }
     p.f[HY][c] = h;
     if (i == p.port_pos[0]) capture(p, s, 0, 1, j, h);
@@ -686,23 +717,23 @@ __device__ __forceinline__ void te2_e_cell(const Params<T> &p, int i, int j, int
   if (i > p.ib && i < p.ie && j >= p.jb && j < p.je) {  // update_ex :43-49
     const T cb = p.cb[0][c];
     const T dhz = A::sub(Hz[c + 1], Hz[c]);
-    T e = A::add(p.f[EX][c], A::div(A::mul(cb, dhz), p.kd[1][j], p.rkd[1][j]));
+    T e = A::step(p.f[EX][c], cb, dhz, p.kd[1][j], p.rkd[1][j]);
     if ((q = e_slab(j, p.jb, p.je, P, d, side)) >= 0) {   // update_pml_ex_yinc :79-87
       T *ps = p.psi[EX][AY][side] + (long long)i * P + d;
-      T v = A::add(A::mul(p.be[q], *ps), A::div(A::mul(p.ce[q], dhz), p.dx, p.rdx));
+      T v = A::psi(p.be[q], *ps, p.ce[q], dhz, p.dx, p.rdx);
       *ps = v;
-      e = A::add(e, A::mul(cb, v));
+      e = A::inc(e, cb, v);
     }
     p.f[EX][c] = e;
   }
   if (i >= p.ib && i < p.ie && j > p.jb && j < p.je) {  // update_ey :52-58
     const T cb = p.cb[1][c];
-    T e = A::add(p.f[EY][c], A::div(A::mul(cb, A::sub(Hz[c], Hz[c + ny])), p.kd[0][i], p.rkd[0][i]));
+    T e = A::step(p.f[EY][c], cb, A::sub(Hz[c], Hz[c + ny]), p.kd[0][i], p.rkd[0][i]);
     if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {   // update_pml_ey_xinc :91-99
       T *ps = p.psi[EY][AX][side] + (long long)d * ny + j;
-      T v = A::add(A::mul(p.be[q], *ps), A::div(A::mul(p.ce[q], A::sub(Hz[c + ny], Hz[c])), p.dx, p.rdx));
+      T v = A::psi(p.be[q], *ps, p.ce[q], A::sub(Hz[c + ny], Hz[c]), p.dx, p.rdx);
       *ps = v;
-      e = A::sub(e, A::mul(cb, v));
+      e = A::dec(e, cb, v);
     }
     p.f[EY][c] = e;
     if (i == p.port_pos[0]) capture(p, s, 0, 0, j, e);
@@ -721,20 +752,19 @@ __device__ __forceinline__ void te2_h_cell(const Params<T> &p, int i, int j, int
   if (i > p.ib && i < p.ie && j > p.jb && j < p.je) {  // update_hz :61-67
     const T dex = A::sub(Ex[c], Ex[c - 1]);
     const T dey = A::sub(Ey[c], Ey[c - ny]);
-    T h = A::add(p.f[HZ][c], A::mul(db, A::sub(A::div(dex, p.kd[4][j], p.rkd[4][j]),
-                                                A::div(dey, p.kd[3][i], p.rkd[3][i]))));
+    T h = A::curl(p.f[HZ][c], db, dex, p.kd[4][j], p.rkd[4][j], dey, p.kd[3][i], p.rkd[3][i]);
     if (in_src(p, HZ, i, j, 0)) h = A::sub(h, p.jsrc[n]);  // source after update_hz
     if ((q = h_slab(i, p.ib, p.ie, P, d, side)) >= 0) {     // update_pml_hz_xinc :103-111
       T *ps = p.psi[HZ][AX][side] + (long long)d * ny + j;
-      T v = A::add(A::mul(p.bh[q], *ps), A::div(A::mul(p.ch[q], dey), p.dx, p.rdx));
+      T v = A::psi(p.bh[q], *ps, p.ch[q], dey, p.dx, p.rdx);
       *ps = v;
-      h = A::sub(h, A::mul(db, v));
+      h = A::dec(h, db, v);
     }
     if ((q = h_slab(j, p.jb, p.je, P, d, side)) >= 0) {     // update_pml_hz_yinc :115-123
       T *ps = p.psi[HZ][AY][side] + (long long)i * P + d;
-      T v = A::add(A::mul(p.bh[q], *ps), A::div(A::mul(p.ch[q], dex), p.dx, p.rdx));
+      T v = A::psi(p.bh[q], *ps, p.ch[q], dex, p.dx, p.rdx);
       *ps = v;
-      h = A::add(h, A::mul(db, v));
+      h = A::inc(h, db, v);
     }
     p.f[HZ][c] = h;
     if (i == p.port_pos[0]) capture(p, s, 0, 1, j, h);

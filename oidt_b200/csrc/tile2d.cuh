@@ -1,4 +1,5 @@
-// tile2d.cuh -- 2D TM / TE time steps, temporally blocked in tiles.
+// tile2d.cuh -- 2D TM / TE time steps, temporally blocked in tiles: float64 and
+// EXACT runs (float32 fast runs: strip2d.cuh).
 //
 // A 2D job of the served sizes (a few hundred x a few hundred cells) is too
 // small to fill the GPU, so with one launch per half-step its step time is
@@ -241,17 +242,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
         if (fl & kE1) {  // update_ez :44-49
           const T dhy = A::sub(F2[t + ncol], f2);
           const T dhx = A::sub(F1[t + 1], f1);
-          T e = A::add(f0, A::mul(cbA, A::sub(A::div(dhy, kr[0], kr[RM]), A::div(dhx, kc[0], kc[CM]))));
+          T e = A::curl(f0, cbA, dhy, kr[0], kr[RM], dhx, kc[0], kc[CM]);
           if (fl & kSrc) e = A::sub(e, __ldg(p.jsrc + n0 + s));  // update_source :71-76
           if (fl & kXE) {                                        // update_pml_ez_xinc :80-88
             const int q = (qE & 0xffff) - 1;
-            xe = A::add(A::mul(BE[q], xe), A::div(A::mul(CE[q], dhy), p.dx, p.rdx));
-            e = A::add(e, A::mul(cbA, xe));
+            xe = A::psi(BE[q], xe, CE[q], dhy, p.dx, p.rdx);
+            e = A::inc(e, cbA, xe);
           }
           if (fl & kYE) {                                        // update_pml_ez_yinc :92-100
             const int q = (qE >> 16) - 1;
-            ye = A::add(A::mul(BE[q], ye), A::div(A::mul(CE[q], dhx), p.dx, p.rdx));
-            e = A::sub(e, A::mul(cbA, ye));
+            ye = A::psi(BE[q], ye, CE[q], dhx, p.dx, p.rdx);
+            e = A::dec(e, cbA, ye);
           }
           f0 = e;
           F0[t] = e;
@@ -261,22 +262,22 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
       } else {
         if (fl & kE1) {  // update_ex :43-49
           const T dhz = A::sub(F2[t + 1], f2);
-          T e = A::add(f0, A::div(A::mul(cbA, dhz), kc[0], kc[CM]));
+          T e = A::step(f0, cbA, dhz, kc[0], kc[CM]);
           if (fl & kYE) {                                        // update_pml_ex_yinc :79-87
             const int q = (qE >> 16) - 1;
-            ye = A::add(A::mul(BE[q], ye), A::div(A::mul(CE[q], dhz), p.dx, p.rdx));
-            e = A::add(e, A::mul(cbA, ye));
+            ye = A::psi(BE[q], ye, CE[q], dhz, p.dx, p.rdx);
+            e = A::inc(e, cbA, ye);
           }
           f0 = e;
           F0[t] = e;
         }
         if (fl & kE2) {  // update_ey :52-58
           const T hz1 = F2[t + ncol];
-          T e = A::add(f1, A::div(A::mul(cbB, A::sub(f2, hz1)), kr[0], kr[RM]));
+          T e = A::step(f1, cbB, A::sub(f2, hz1), kr[0], kr[RM]);
           if (fl & kXE) {                                        // update_pml_ey_xinc :91-99
             const int q = (qE & 0xffff) - 1;
-            xe = A::add(A::mul(BE[q], xe), A::div(A::mul(CE[q], A::sub(hz1, f2)), p.dx, p.rdx));
-            e = A::sub(e, A::mul(cbB, xe));
+            xe = A::psi(BE[q], xe, CE[q], A::sub(hz1, f2), p.dx, p.rdx);
+            e = A::dec(e, cbB, xe);
           }
           f1 = e;
           F1[t] = e;
@@ -289,22 +290,22 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
       if (TM) {
         if (fl & kH1) {  // update_hx :53-58
           const T ezm = F0[t - 1];
-          T h = A::add(f1, A::div(A::mul(db, A::sub(ezm, f0)), kc[2 * CM], kc[3 * CM]));
+          T h = A::step(f1, db, A::sub(ezm, f0), kc[2 * CM], kc[3 * CM]);
           if (fl & kYH) {                                        // update_pml_hx_yinc :104-112
             const int q = (qH >> 16) - 1;
-            yh = A::add(A::mul(BH[q], yh), A::div(A::mul(CH[q], A::sub(f0, ezm)), p.dx, p.rdx));
-            h = A::sub(h, A::mul(db, yh));
+            yh = A::psi(BH[q], yh, CH[q], A::sub(f0, ezm), p.dx, p.rdx);
+            h = A::dec(h, db, yh);
           }
           f1 = h;
           F1[t] = h;
         }
         if (fl & kH2) {  // update_hy :62-67
           const T dez = A::sub(f0, F0[t - ncol]);
-          T h = A::add(f2, A::div(A::mul(db, dez), kr[2 * RM], kr[3 * RM]));
+          T h = A::step(f2, db, dez, kr[2 * RM], kr[3 * RM]);
           if (fl & kXH) {                                        // update_pml_hy_xinc :116-124
             const int q = (qH & 0xffff) - 1;
-            xh = A::add(A::mul(BH[q], xh), A::div(A::mul(CH[q], dez), p.dx, p.rdx));
-            h = A::add(h, A::mul(db, xh));
+            xh = A::psi(BH[q], xh, CH[q], dez, p.dx, p.rdx);
+            h = A::inc(h, db, xh);
           }
           f2 = h;
           F2[t] = h;
@@ -315,17 +316,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
         if (fl & kH1) {  // update_hz :61-67
           const T dex = A::sub(f0, F0[t - 1]);
           const T dey = A::sub(f1, F1[t - ncol]);
-          T h = A::add(f2, A::mul(db, A::sub(A::div(dex, kc[2 * CM], kc[3 * CM]), A::div(dey, kr[2 * RM], kr[3 * RM]))));
+          T h = A::curl(f2, db, dex, kc[2 * CM], kc[3 * CM], dey, kr[2 * RM], kr[3 * RM]);
           if (fl & kSrc) h = A::sub(h, __ldg(p.jsrc + n0 + s));  // source after update_hz
           if (fl & kXH) {                                        // update_pml_hz_xinc :103-111
             const int q = (qH & 0xffff) - 1;
-            xh = A::add(A::mul(BH[q], xh), A::div(A::mul(CH[q], dey), p.dx, p.rdx));
-            h = A::sub(h, A::mul(db, xh));
+            xh = A::psi(BH[q], xh, CH[q], dey, p.dx, p.rdx);
+            h = A::dec(h, db, xh);
           }
           if (fl & kYH) {                                        // update_pml_hz_yinc :115-123
             const int q = (qH >> 16) - 1;
-            yh = A::add(A::mul(BH[q], yh), A::div(A::mul(CH[q], dex), p.dx, p.rdx));
-            h = A::add(h, A::mul(db, yh));
+            yh = A::psi(BH[q], yh, CH[q], dex, p.dx, p.rdx);
+            h = A::inc(h, db, yh);
           }
           f2 = h;
           F2[t] = h;
