@@ -344,11 +344,11 @@ long long psi_elems(int mode, int axis, int nx, int ny, int nz, int P, int pitch
   return (long long)nx * ny * (zpitch > 0 ? zpitch : P);
 }
 
-// The vector form's z-slab psi rows.  A row holds every four-cell group that
+// The vector form's z-slab psi rows.  A row holds every group of four cells that
 // meets the slab: slab cell d of the low side (k = kb + d) sits at
 // zoff[LO] + d = k - floor4(kb), of the high side (k = ke - P + d) at
 // zoff[HI] + d = k - floor4(ke - P).  A group k0 of the slab's groups then
-// reads its four values at one 16-byte aligned offset, k0 - floor4(start).
+// (in float64, each half of it) reads its values at one 16-byte aligned offset, k0 - floor4(start).
 struct ZRows {
   int pitch, off[2];
 };
@@ -447,26 +447,27 @@ int choose_chunk(const oidt_job_desc *d, int slots) {
 
 int g_sweep_slots = 0;  // SMs x resident sweep CTAs (set at context creation)
 
-// Split of a 3D row between the vector form's roles: four-cell groups over
+// Split of a 3D row between the vector form's roles: groups of W (4 or 2) cells over
 // k in [kb + P, ke - P) rounded inward to multiples of 4 (vector role), the
-// other four-cell groups of the row (edge role).
-VecGeom vec_geom_of(int kb, int ke, int P, int jb, int je, int nzp) {
+// other groups of the row (edge role).
+VecGeom vec_geom_of(int kb, int ke, int P, int jb, int je, int nzp, int W) {
   VecGeom g;
   g.kz0 = (kb + P + 3) / 4 * 4;
   g.kz1 = (ke - P) / 4 * 4;
   if (g.kz1 <= g.kz0) g.kz0 = g.kz1 = nzp;  // no z-clean group: every cell in the edge role
-  g.nvc = (g.kz1 - g.kz0) / 4;
+  g.nvc = (g.kz1 - g.kz0) / W;
   g.nedge = g.kz0 + (nzp - g.kz1);
   const long long rows = je - jb;
   g.nb_vec = (int)((rows * g.nvc + kVecThreads - 1) / kVecThreads);
   return g;
 }
-int vec_edge_blocks(const VecGeom &g, int jb, int je) {
-  return (int)(((long long)(je - jb) * (g.nedge / 4) + kVecThreads - 1) / kVecThreads);
+int vec_edge_blocks(const VecGeom &g, int jb, int je, int W) {
+  return (int)(((long long)(je - jb) * (g.nedge / W) + kVecThreads - 1) / kVecThreads);
 }
+// of the ordered form
 long long vec_blocks_per_plane(const oidt_job_desc *d, int nzp) {
-  const VecGeom g = vec_geom_of(d->kb, d->ke, d->num_cpml, d->jb, d->je, nzp);
-  return (long long)g.nb_vec + vec_edge_blocks(g, d->jb, d->je);
+  const VecGeom g = vec_geom_of(d->kb, d->ke, d->num_cpml, d->jb, d->je, nzp, 4);
+  return (long long)g.nb_vec + vec_edge_blocks(g, d->jb, d->je, 4);
 }
 
 int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
@@ -960,13 +961,15 @@ void y3_half(int rows, bool H, bool pdl, const Params<T> &p, int s, cudaStream_t
   else y3_half_by<T, EXACT, 4>(H, pdl, p, s, st);
 }
 
-template <typename T> VecGeom vec_geom(const Params<T> &p) { return vec_geom_of(p.kb, p.ke, p.P, p.jb, p.je, p.nzp); }
+template <typename T> VecGeom vec_geom(const Params<T> &p, int W) {
+  return vec_geom_of(p.kb, p.ke, p.P, p.jb, p.je, p.nzp, W);
+}
 
 // One 3D vector-form half-step: the vector-role blocks, then the edge-role
 // blocks, of one x-plane per grid row.
 template <typename T, bool EXACT> void v3_half(bool H, bool pdl, const Params<T> &p, int s, cudaStream_t st) {
-  const VecGeom g = vec_geom(p);
-  const long long nb_edge = vec_edge_blocks(g, p.jb, p.je);
+  const VecGeom g = vec_geom(p, kVecW<T>);
+  const long long nb_edge = vec_edge_blocks(g, p.jb, p.je, kVecW<T>);
   const dim3 grd((unsigned)(g.nb_vec + nb_edge), p.ie - p.ib), blk(kVecThreads);
   void (*kern)(Params<T>, VecGeom, int) = H ? k_v3_h<T, EXACT> : k_v3_e<T, EXACT>;
   if (pdl) launch_step_kernel(kern, grd, blk, 0, st, p, g, s);
@@ -984,10 +987,10 @@ template <typename T> int wave_lag(const Params<T> &p) {
 }
 
 template <typename T, bool EXACT> void v3_wave(Job *J, bool pdl, const Params<T> &p, int s, cudaStream_t st) {
-  const VecGeom g = vec_geom(p);
+  const VecGeom g = vec_geom(p, 4);
   WaveArgs w;
   w.done = reinterpret_cast<int *>(J->mem + J->pl.off_wave + 8);
-  w.nb = g.nb_vec + vec_edge_blocks(g, p.jb, p.je);
+  w.nb = g.nb_vec + vec_edge_blocks(g, p.jb, p.je, 4);
   w.lag = wave_lag(p);
   const dim3 grd((unsigned)(2LL * (p.ie - p.ib) * w.nb)), blk(kVecThreads);
   if (pdl) launch_step_kernel(k_v3_wave<T, EXACT>, grd, blk, 0, st, p, g, w, s);

@@ -36,6 +36,11 @@ enum { LO = 0, HI = 1 };
 // the numerator, the quotient and the reciprocal stay within [2^-lo, 2^lo]
 // (the residuals are then exact); outside that range, and for NaN, the
 // quotient is divided directly.  Zero numerators give a zero of either sign.
+// quo() is the same quotient with the range left to the caller, who divides a
+// whole group's quotients directly (ieee) if any is out of range: `in` tests a
+// numerator and `yin` a reciprocal by their exponent fields, on the integer
+// pipe and before the quotients (seven FP64 comparisons and a branch a
+// quotient weighed more than its five FP64 operations).
 template <typename T, bool EXACT> struct Ar;
 template <> struct Ar<float, true> {
   static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
@@ -48,6 +53,16 @@ template <> struct Ar<float, true> {
                     ay >= 0x1p-100f && ay <= 0x1p+100f;
     if (!ok) return __fdiv_rn(a, b);
     const float q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
+    return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
+  }
+  static __device__ __forceinline__ float ieee(float a, float b) { return __fdiv_rn(a, b); }
+  static __device__ __forceinline__ bool in(float a) {  // 0, or 2^-100 <= |a| <= 2^70
+    const unsigned h = __float_as_uint(a) << 1;
+    return h - (27u << 24) <= (170u << 24) || h == 0u;
+  }
+  static __device__ __forceinline__ bool yin(float y) { return (__float_as_uint(y) << 1) - (107u << 24) <= (70u << 24); }  // 2^-20 .. 2^50
+  static __device__ __forceinline__ float quo(float a, float b, float y) {
+    const float q0 = __fmul_rn(a, y), q1 = __fmaf_rn(__fmaf_rn(-b, q0, a), y, q0);
     return __fmaf_rn(__fmaf_rn(-b, q1, a), y, q1);
   }
   // composite operations of an update, as the reference evaluates them
@@ -84,6 +99,18 @@ template <> struct Ar<double, true> {
                     ay >= 0x1p-900 && ay <= 0x1p+900;
     if (!ok) return __ddiv_rn(a, b);
     const double q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    return __fma_rn(__fma_rn(-b, q1, a), y, q1);
+  }
+  static __device__ __forceinline__ double ieee(double a, double b) { return __ddiv_rn(a, b); }
+  static __device__ __forceinline__ bool in(double a) {  // 0, or 2^-800 <= |a| <= 2^800: a y is then in range for any y of yin
+    const unsigned h = (unsigned)__double2hiint(a) << 1;
+    return h - (223u << 21) <= (1600u << 21) || (h | (unsigned)__double2loint(a)) == 0u;
+  }
+  static __device__ __forceinline__ bool yin(double y) {  // 2^-100 .. 2^100
+    return ((unsigned)__double2hiint(y) << 1) - (923u << 21) <= (200u << 21);
+  }
+  static __device__ __forceinline__ double quo(double a, double b, double y) {
+    const double q0 = __dmul_rn(a, y), q1 = __fma_rn(__fma_rn(-b, q0, a), y, q0);
     return __fma_rn(__fma_rn(-b, q1, a), y, q1);
   }
   // composite operations of an update, as the reference evaluates them
