@@ -371,7 +371,7 @@ struct JobPlan {
   size_t off_wave;                // ordered form: E-block counts per plane (after 8 spare bytes)
   size_t off_tile;                // 2D tile form: sub-blocks completed per tile [kTileMaxBlocks] ...
   bool strip;                     // ... the strip kernel (float32 fast; else one cell a thread) ...
-  size_t off_xch, xch_words;      // ... and its exchange words (0: none)
+  size_t off_xch, xch_words;      // ... and exchange words (0: none)
   size_t off_pow;                 // port power [nf] complex float64
   long long N, plane;
   int K, KL, esz, nzp, nbuf, variant, L, nitems;  // K: steps of a ring block; KL: of a long block (K but for the tile form)
@@ -604,10 +604,12 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
   if (variant == kVariantWave) pl->off_wave = L.take(8 + (size_t)4 * (d->ie - d->ib));
   if (variant == kVariantTile) {
     pl->off_tile = L.take((size_t)4 * kTileMaxBlocks);
-    // the strip kernel's exchange words (34 MB at most), for grids a cooperative launch can hold
+    // exchange words (34 MB at most), for grids a cooperative launch can hold
     pl->strip = d->precision == OIDT_F32 && d->arith == OIDT_ARITH_FAST;
-    pl->xch_words = pl->strip && d->reserved[2] == 0 && N <= kStripCoopCells && (long long)P * (d->nx + d->ny) <= kStripCoopCells
-                        ? 2 * strip2d_xch_buf(d->nx, d->ny, P) : 0;
+    const long long most = pl->strip ? kStripCoopCells : 148LL * kTileThreads;
+    pl->xch_words = d->reserved[2] != 0 || N > most || (long long)P * (d->nx + d->ny) > most ? 0
+                    : pl->strip ? 2 * strip2d_xch_buf(d->nx, d->ny, P)
+                                : 2 * tile2d_xch_buf(esz, d->nx, d->ny, P);
     pl->off_xch = L.take(8 * pl->xch_words);
   }
   if (d->probe[0] == 1) {
@@ -1040,23 +1042,23 @@ void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStre
     a.xbuf = (long long)J->pl.xch_words / 2;
     tile_launch_as(p.mode == OIDT_MODE_TM2 ? strip_kernel<OIDT_MODE_TM2>(a.cells) : strip_kernel<OIDT_MODE_TE2>(a.cells),
                    cnt > a.halo, pdl, J->tile_blocks, a.threads, J->tile_smem, st, p, a);
-    return;
+  } else {
+    void (*kern)(const Params<T>, TileArgs) =
+        p.mode == OIDT_MODE_TM2 ? k_2d_tile<T, EXACT, OIDT_MODE_TM2> : k_2d_tile<T, EXACT, OIDT_MODE_TE2>;
+    TileArgs a = J->tile;
+    a.s0 = s0;
+    a.cnt = cnt;
+    a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
+    a.xch = reinterpret_cast<unsigned long long *>(J->mem + J->pl.off_xch);
+    a.xbuf = (long long)J->pl.xch_words / 2;
+    tile_launch_as(kern, cnt > a.halo, pdl, J->tile_blocks, kTileThreads, J->tile_smem, st, p, a);
   }
-  void (*kern)(Params<T>, TileArgs) =
-      p.mode == OIDT_MODE_TM2 ? k_2d_tile<T, EXACT, OIDT_MODE_TM2> : k_2d_tile<T, EXACT, OIDT_MODE_TE2>;
-  TileArgs a = J->tile;
-  a.s0 = s0;
-  a.cnt = cnt;
-  a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
-  tile_launch_as(kern, cnt > a.halo, pdl, J->tile_blocks, kTileThreads, J->tile_smem, st, p, a);
 }
 
-// Launches of the 2D tile form for cnt steps: up to halo steps each -- also the
-// buffer flips of k_2d_tile's cooperative launch; k_2d_strip's is one flip.
+// Launches of the 2D tile form for cnt steps, each one flip of the buffers:
+// one cooperative launch, or up to halo steps each.
 int tile_halo(const Job *J) { return J->pl.strip ? J->strip.halo : J->tile.halo; }
-int tile_launches(const Job *J, int cnt) {
-  return J->pl.strip && J->tile_coop ? 1 : (cnt + tile_halo(J) - 1) / tile_halo(J);
-}
+int tile_launches(const Job *J, int cnt) { return J->tile_coop ? 1 : (cnt + tile_halo(J) - 1) / tile_halo(J); }
 
 template <typename T> size_t sweep_smem() { return sweep_smem_bytes<T, EYB, EZB, ST>(); }
 
@@ -1435,11 +1437,9 @@ template <typename T, bool EXACT, int MODE> void tile_attrs_of() {
 }
 
 void set_tile_attrs() {
-  tile_attrs_of<float, false, OIDT_MODE_TM2>();
   tile_attrs_of<float, true, OIDT_MODE_TM2>();
   tile_attrs_of<double, false, OIDT_MODE_TM2>();
   tile_attrs_of<double, true, OIDT_MODE_TM2>();
-  tile_attrs_of<float, false, OIDT_MODE_TE2>();
   tile_attrs_of<float, true, OIDT_MODE_TE2>();
   tile_attrs_of<double, false, OIDT_MODE_TE2>();
   tile_attrs_of<double, true, OIDT_MODE_TE2>();
@@ -1713,7 +1713,7 @@ int32_t oidt_job_create(oidt_ctx *ctx, const oidt_job_desc *desc, uint64_t *job)
       J->tile_smem = tile2d_smem(pl.esz, desc->num_cpml, J->tile.ti + 2 * J->tile.halo, J->tile.tj + 2 * J->tile.halo);
       // a ring block in one launch where every tile is resident at once and a tile's
       // halo reaches its 8 neighbours only
-      J->tile_coop = ctx->coop && desc->reserved[2] == 0 && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
+      J->tile_coop = ctx->coop && pl.xch_words > 0 && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
                      J->tile.halo <= std::min(J->tile.ti, J->tile.tj) && J->pl.K > J->tile.halo;
     }
     if (J->tile_blocks == 0) {

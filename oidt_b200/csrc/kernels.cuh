@@ -40,7 +40,8 @@ enum { LO = 0, HI = 1 };
 // whole group's quotients directly (ieee) if any is out of range: `in` tests a
 // numerator and `yin` a reciprocal by their exponent fields, on the integer
 // pipe and before the quotients (seven FP64 comparisons and a branch a
-// quotient weighed more than its five FP64 operations).
+// quotient weighed more than its five FP64 operations: 400 x 200 float64 EXACT
+// 2.62 -> 2.45 us per step).
 template <typename T, bool EXACT> struct Ar;
 template <> struct Ar<float, true> {
   static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
@@ -67,10 +68,19 @@ template <> struct Ar<float, true> {
   }
   // composite operations of an update, as the reference evaluates them
   static __device__ __forceinline__ float curl(float e, float c, float a, float ka, float ra, float b, float kb, float rb) {
-    return add(e, mul(c, sub(div(a, ka, ra), div(b, kb, rb))));
+    float qa, qb;
+    if (in(a) & in(b) & yin(ra) & yin(rb)) {
+      qa = quo(a, ka, ra);
+      qb = quo(b, kb, rb);
+    } else {
+      qa = ieee(a, ka);
+      qb = ieee(b, kb);
+    }
+    return add(e, mul(c, sub(qa, qb)));
   }
-  static __device__ __forceinline__ float step(float e, float c, float d, float k, float r) { return add(e, div(mul(c, d), k, r)); }
-  static __device__ __forceinline__ float psi(float b, float q, float c, float d, float k, float r) { return add(mul(b, q), div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ float divi(float a, float b, float y) { return in(a) & yin(y) ? quo(a, b, y) : ieee(a, b); }
+  static __device__ __forceinline__ float step(float e, float c, float d, float k, float r) { return add(e, divi(mul(c, d), k, r)); }
+  static __device__ __forceinline__ float psi(float b, float q, float c, float d, float k, float r) { return add(mul(b, q), divi(mul(c, d), k, r)); }
   static __device__ __forceinline__ float inc(float e, float c, float q) { return add(e, mul(c, q)); }
   static __device__ __forceinline__ float dec(float e, float c, float q) { return sub(e, mul(c, q)); }
 };
@@ -115,10 +125,19 @@ template <> struct Ar<double, true> {
   }
   // composite operations of an update, as the reference evaluates them
   static __device__ __forceinline__ double curl(double e, double c, double a, double ka, double ra, double b, double kb, double rb) {
-    return add(e, mul(c, sub(div(a, ka, ra), div(b, kb, rb))));
+    double qa, qb;
+    if (in(a) & in(b) & yin(ra) & yin(rb)) {
+      qa = quo(a, ka, ra);
+      qb = quo(b, kb, rb);
+    } else {
+      qa = ieee(a, ka);
+      qb = ieee(b, kb);
+    }
+    return add(e, mul(c, sub(qa, qb)));
   }
-  static __device__ __forceinline__ double step(double e, double c, double d, double k, double r) { return add(e, div(mul(c, d), k, r)); }
-  static __device__ __forceinline__ double psi(double b, double q, double c, double d, double k, double r) { return add(mul(b, q), div(mul(c, d), k, r)); }
+  static __device__ __forceinline__ double divi(double a, double b, double y) { return in(a) & yin(y) ? quo(a, b, y) : ieee(a, b); }
+  static __device__ __forceinline__ double step(double e, double c, double d, double k, double r) { return add(e, divi(mul(c, d), k, r)); }
+  static __device__ __forceinline__ double psi(double b, double q, double c, double d, double k, double r) { return add(mul(b, q), divi(mul(c, d), k, r)); }
   static __device__ __forceinline__ double inc(double e, double c, double q) { return add(e, mul(c, q)); }
   static __device__ __forceinline__ double dec(double e, double c, double q) { return sub(e, mul(c, q)); }
 };

@@ -56,7 +56,7 @@
 // with the same operations and never written back.
 #pragma once
 
-#include "kernels.cuh"
+#include "tile2d.cuh"
 
 namespace oidt {
 
@@ -87,35 +87,6 @@ inline size_t strip2d_smem(int rows, int cols, int C, int steps) {
 // Exchange words of a job (64-bit), two buffers of: f0, f1 [nx ny][2], x-slab
 // psi of E, H [side][P][ny][2], y-slab psi [side][nx][P][2], f2 [nx ny].
 inline size_t strip2d_xch_buf(long long nx, long long ny, long long P) { return (size_t)((3 * nx * ny + 4 * P * (nx + ny) + 1) / 2 * 2); }
-
-// Two values, each beside the number n, to q[0..1].
-__device__ __forceinline__ void xch_put(unsigned long long *q, float v0, float v1, unsigned n) {
-  const unsigned long long h = (unsigned long long)n << 32;
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(q), "l"(h | __float_as_uint(v0)),
-               "l"(h | __float_as_uint(v1))
-               : "memory");
-}
-__device__ __forceinline__ void xch_put(unsigned long long *q, float v, unsigned n) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(q), "l"((unsigned long long)n << 32 | __float_as_uint(v))
-               : "memory");
-}
-// Predicated: q[0..1], or q[0], is loaded where `on`, else w is left.
-__device__ __forceinline__ void xch_load(unsigned long long &w, const unsigned long long *q, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.relaxed.gpu.global.b64 %0, [%1];\n}\n"
-               : "+l"(w)
-               : "l"(q), "r"((unsigned)on)
-               : "memory");
-}
-__device__ __forceinline__ void xch_load2(unsigned long long *w, const unsigned long long *q, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];\n}\n"
-               : "+l"(w[0]), "+l"(w[1])
-               : "l"(q), "r"((unsigned)on)
-               : "memory");
-}
-__device__ __forceinline__ bool xch_take(unsigned long long w, float &v, unsigned n, bool on) {
-  v = on ? __uint_as_float((unsigned)w) : v;
-  return !on || (unsigned)(w >> 32) == n;
-}
 
 // Cell flags.  TM: E1 = Ez update, H1 = Hx, H2 = Hy; TE: E1 = Ex, E2 = Ey,
 // H1 = Hz.  XE / YE / XH / YH: the cell's component is in the E / H x- /

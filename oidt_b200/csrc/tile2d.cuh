@@ -22,21 +22,26 @@
 //   thread), the CPML coefficient tables, and the kappa dx divisors with
 //   their reciprocals for the tile's rows and columns; __syncthreads
 //   separates the half-steps.
-// * Fields and psi are double-buffered: sub-block b reads the state of
-//   buffer par ^ (b & 1) and writes its owned cells to the other, so blocks
-//   loading halo cells never see cells another block has already advanced.
-// * A launch of one sub-block (cnt <= halo) needs no other synchronisation:
-//   a grid with more tiles than SMs simply runs in waves.  A launch of
-//   several sub-blocks is cooperative (all tiles resident at once): before
-//   sub-block b > 0 a block waits until each of its (up to 8) neighbour tiles
-//   has published, through its counter in `epoch` (release / acquire), that
-//   it finished sub-block b - 1 -- its owned cells written, its reads of the
-//   buffer this block writes next done.  Halo width <= tile extent, so no
-//   other tile's cells are read.  The wait is bounded (p.wait_cycles); on
-//   expiry the block records state[1] = 3 and goes on.  Between sub-blocks
-//   only what other tiles read crosses global memory: a tile stores its owned
-//   cells within `halo` of its edges and reloads its halo cells; the other
-//   owned cells stay in registers (and are stored after the last sub-block).
+// * A launch of one sub-block (cnt <= halo) reads one field / psi buffer and
+//   writes its owned cells to the other, so no block sees cells another has
+//   advanced; a grid with more tiles than SMs simply runs in waves.
+// * A launch of several sub-blocks is cooperative (all tiles resident at
+//   once).  Between sub-blocks only what other tiles read moves: a tile puts
+//   its owned cells within `halo` of its edges (fields and psi) into the
+//   exchange words and polls its halo cells' words, which their tiles (up to
+//   8, as halo width <= tile extent) put there; everything else stays in
+//   registers, and the owned cells are stored once, after the last sub-block.
+//   Two buffers of words alternate: a tile writes sub-block b + 1's words over
+//   those of b - 1 only after it has read its neighbours' b, which they put
+//   after reading its b - 1.  Each wait is bounded (p.wait_cycles); on expiry
+//   the block records state[1] = 3 and goes on without waiting again.
+//
+// What bounds it: latency -- two block barriers and a dependent chain a step,
+// an L2 store and load a crossing.  A crossing through the field buffers
+// behind per-tile counters (fence, release, acquire, then the loads) took 3.5 us
+// where the words take 2.1.  Measured on a B200, 400 x 200 float64 in sub-blocks
+// of 4: EXACT 2.95 -> 2.62 us per step with the words, -> 2.45 with the range
+// test on the integer pipe (kernels.cuh, Ar); fast 2.08 -> 1.97.
 //
 // Per cell the arithmetic is that of kernels.cuh's tm2_e_cell / tm2_h_cell /
 // te2_e_cell / te2_h_cell (the reference's fdtd_funcs.py of FDTD_2D_TM and
@@ -59,7 +64,62 @@ struct TileArgs {
   int gj;      // tiles along y
   int halo;    // cells computed on each side of the owned tile; steps per sub-block
   int *epoch;  // per tile: sub-blocks completed (cooperative launches)
+  unsigned long long *xch;  // exchange words, two buffers ...
+  long long xbuf;           // ... of xbuf words
 };
+
+// Exchange words (64 bits: 32 bits of a value beside the 32-bit number of the
+// sub-block that wrote it).  A 64-bit access is single-copy atomic, so the
+// reader polls the data word itself until the number is the one it waits for;
+// no fence, flag or barrier orders data against a flag.  A float32 value is one
+// word, a float64 value two.
+__device__ __forceinline__ void xch_put(unsigned long long *q, float v0, float v1, unsigned n) {  // two values to q[0..1]
+  const unsigned long long h = (unsigned long long)n << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(q), "l"(h | __float_as_uint(v0)),
+               "l"(h | __float_as_uint(v1))
+               : "memory");
+}
+__device__ __forceinline__ void xch_put(unsigned long long *q, float v, unsigned n) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(q), "l"((unsigned long long)n << 32 | __float_as_uint(v))
+               : "memory");
+}
+__device__ __forceinline__ void xch_put(unsigned long long *q, double v, unsigned n) {  // to q[0..1]
+  const unsigned long long h = (unsigned long long)n << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(q), "l"(h | (unsigned)__double2loint(v)),
+               "l"(h | (unsigned)__double2hiint(v))
+               : "memory");
+}
+// Predicated (all loads of a poll are in flight together): q[0..1], or q[0],
+// is loaded where `on`, else w is left.
+__device__ __forceinline__ void xch_load(unsigned long long &w, const unsigned long long *q, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n @p ld.relaxed.gpu.global.b64 %0, [%1];\n}\n"
+               : "+l"(w)
+               : "l"(q), "r"((unsigned)on)
+               : "memory");
+}
+__device__ __forceinline__ void xch_load2(unsigned long long *w, const unsigned long long *q, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];\n}\n"
+               : "+l"(w[0]), "+l"(w[1])
+               : "l"(q), "r"((unsigned)on)
+               : "memory");
+}
+__device__ __forceinline__ bool xch_take(unsigned long long w, float &v, unsigned n, bool on) {
+  v = on ? __uint_as_float((unsigned)w) : v;
+  return !on || (unsigned)(w >> 32) == n;
+}
+// A value's words in tile2d's exchange.
+__device__ __forceinline__ void xch_load(unsigned long long *w, const unsigned long long *q, bool on, float) { xch_load(w[0], q, on); }
+__device__ __forceinline__ void xch_load(unsigned long long *w, const unsigned long long *q, bool on, double) { xch_load2(w, q, on); }
+__device__ __forceinline__ bool xch_take(const unsigned long long *w, float &v, unsigned n, bool on) { return xch_take(w[0], v, n, on); }
+__device__ __forceinline__ bool xch_take(const unsigned long long *w, double &v, unsigned n, bool on) {
+  v = on ? __hiloint2double((int)(unsigned)w[1], (int)(unsigned)w[0]) : v;
+  return !on || ((unsigned)(w[0] >> 32) == n && (unsigned)(w[1] >> 32) == n);
+}
+// Words of one buffer: the three fields [nx ny], x-slab psi of E and H
+// [2 sides][P][ny], y-slab psi of E and H [2 sides][nx][P].
+inline size_t tile2d_xch_buf(int esz, long long nx, long long ny, long long P) {
+  return (size_t)(esz / 4) * (3 * nx * ny + 4 * P * (nx + ny) + (nx * ny & 1));
+}
 
 // Shared memory of a block: the tile's three fields (kTileThreads cells each),
 // the CPML coefficient tables be, ce, bh, ch (P each), and per held row (at
@@ -80,7 +140,7 @@ enum : unsigned {
 };
 
 template <typename T, bool EXACT, int MODE>
-__global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileArgs a) {
+__global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_constant__ Params<T> p, TileArgs a) {
   using A = Ar<T, EXACT>;
   constexpr bool TM = MODE == OIDT_MODE_TM2;
   // fields f0, f1 (E in TE, H in TM), f2 (H); the fields carrying each psi array
@@ -101,7 +161,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
   const int t = threadIdx.x;
   const bool act = t < nrow * ncol;
   const int li = act ? t / ncol : 0, lj = act ? t - li * ncol : 0, i = wi0 + li, j = wj0 + lj;
-  const int g = i * ny + j;  // the cell in the [nx][ny] arrays (2^31 cells at most)
+  int gx = i * ny + j;
+  const int g = gx;  // the cell in the [nx][ny] arrays (2^31 cells at most)
   // ---- the cell's constants ------------------------------------------------------------
   unsigned fl = 0;
   int qE = 0, qH = 0;  // slab coefficient indices + 1: x slab in bits 0-15, y slab in bits 16-31
@@ -198,42 +259,21 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
   const int n0 = p.state[0] + a.s0;
   const int e0 = nsub > 1 ? a.epoch[blockIdx.x] : 0;  // equal for every tile at launch
   T f0 = T(0), f1 = T(0), f2 = T(0), xe = T(0), ye = T(0), xh = T(0), yh = T(0);  // the cell's values
+  if (act) {  // the held tile
+    f0 = __ldcg(p.f[FA] + g);
+    f1 = __ldcg(p.f[FB] + g);
+    f2 = __ldcg(p.f[FC] + g);
+    F0[t] = f0;
+    F1[t] = f1;
+    F2[t] = f2;
+    if (fl & kXE) xe = __ldcg(p.psi[EXS][AX][sides & 1] + oxE);
+    if (fl & kYE) ye = __ldcg(p.psi[EYS][AY][(sides >> 1) & 1] + oyE);
+    if (fl & kXH) xh = __ldcg(p.psi[HXS][AX][(sides >> 2) & 1] + oxH);
+    if (fl & kYH) yh = __ldcg(p.psi[HYS][AY][(sides >> 3) & 1] + oyH);
+  }
+  __syncthreads();
+  bool waits = true;
   for (int sb = 0; sb < nsub; ++sb) {
-    T **rf = (sb & 1) ? p.fn : p.f;  // buffers read and written in this sub-block
-    T **wf = (sb & 1) ? p.f : p.fn;
-    T *(*rp)[3][2] = (sb & 1) ? p.psin : p.psi;
-    T *(*wp)[3][2] = (sb & 1) ? p.psi : p.psin;
-    if (sb > 0) {  // the neighbour tiles have finished sub-block sb - 1
-      if (t < 9 && t != 4) {
-        const int nbi = bi + t / 3 - 1, nbj = bj + t % 3 - 1;
-        const int gi = (nx + a.ti - 1) / a.ti;
-        if (nbi >= 0 && nbi < gi && nbj >= 0 && nbj < a.gj) {
-          const int *ep = a.epoch + nbi * a.gj + nbj;
-          const long long t0 = clock64();
-          while (ld_acquire(ep) < e0 + sb) {
-            if (clock64() - t0 > p.wait_cycles) {
-              atomicExch(p.state + 1, 3);  // reported to the host by oidt_job_sync
-              break;
-            }
-            if (ld_acquire(p.state + 1) != 0) break;  // an earlier wait expired: stop waiting
-          }
-        }
-      }
-      __syncthreads();
-    }
-    if (act && (sb == 0 || !(fl & kOwn))) {  // the held tile of the buffer read (L2: other blocks wrote it)
-      f0 = __ldcg(rf[FA] + g);
-      f1 = __ldcg(rf[FB] + g);
-      f2 = __ldcg(rf[FC] + g);
-      F0[t] = f0;
-      F1[t] = f1;
-      F2[t] = f2;
-      if (fl & kXE) xe = __ldcg(rp[EXS][AX][sides & 1] + oxE);
-      if (fl & kYE) ye = __ldcg(rp[EYS][AY][(sides >> 1) & 1] + oyE);
-      if (fl & kXH) xh = __ldcg(rp[HXS][AX][(sides >> 2) & 1] + oxH);
-      if (fl & kYH) yh = __ldcg(rp[HYS][AY][(sides >> 3) & 1] + oyH);
-    }
-    __syncthreads();
     const int s1 = min(a.cnt, (sb + 1) * H);
     for (int s = sb * H; s < s1; ++s) {
       T *const ring = p.ring + (a.s0 + s) * cstride;  // the step's ring slot
@@ -336,24 +376,71 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(Params<T> p, TileAr
       }
       __syncthreads();
     }
-    // ---- owned cells to the buffer written (before the last sub-block: those other tiles read)
-    if ((fl & kOwn) && (sb == nsub - 1 || (fl & kBand))) {
-      wf[FA][g] = f0;
-      wf[FB][g] = f1;
-      wf[FC][g] = f2;
-      if (fl & kXE) wp[EXS][AX][sides & 1][oxE] = xe;
-      if (fl & kYE) wp[EYS][AY][(sides >> 1) & 1][oyE] = ye;
-      if (fl & kXH) wp[HXS][AX][(sides >> 2) & 1][oxH] = xh;
-      if (fl & kYH) wp[HYS][AY][(sides >> 3) & 1][oyH] = yh;
+    if (sb == nsub - 1) break;
+    // ---- between sub-blocks: put the owned cells other tiles hold, fetch the halo cells ----
+    const unsigned n = (unsigned)(e0 + sb + 1);
+    asm volatile("" : "+r"(gx), "+r"(sides));  // the words' places are formed here, not held through the steps
+    constexpr int XW = (int)sizeof(T) / 4;
+    const int N = nx * ny, SX = 2 * P * ny, SY = 2 * nx * P;
+    unsigned long long *const xb = a.xch + ((n & 1) ? a.xbuf : 0);
+    auto word = [&](int v) { return xb + (long long)XW * v; };
+    const int pxe = 3 * N + (sides & 1) * P * ny + oxE, pxh = 3 * N + SX + ((sides >> 2) & 1) * P * ny + oxH;
+    const int pye = 3 * N + 2 * SX + ((sides >> 1) & 1) * nx * P + oyE, pyh = 3 * N + 2 * SX + SY + ((sides >> 3) & 1) * nx * P + oyH;
+    if (fl & kBand) {
+      xch_put(word(gx), f0, n);
+      xch_put(word(N + gx), f1, n);
+      xch_put(word(2 * N + gx), f2, n);
+      if (fl & kXE) xch_put(word(pxe), xe, n);
+      if (fl & kYE) xch_put(word(pye), ye, n);
+      if (fl & kXH) xch_put(word(pxh), xh, n);
+      if (fl & kYH) xch_put(word(pyh), yh, n);
     }
-    if (nsub > 1) {  // publish: this tile finished sub-block sb (the barrier orders every
-      __syncthreads();  // thread's stores before thread 0's fence, which is cumulative)
-      if (t == 0) {
-        __threadfence();
-        st_release(a.epoch + blockIdx.x, e0 + sb + 1);
+    if (act && !(fl & kOwn)) {
+      const long long t0 = clock64();
+      unsigned round = 0;
+      for (;;) {
+        unsigned long long w[4][XW] = {};
+        xch_load(w[0], word(gx), true, T(0));
+        xch_load(w[1], word(N + gx), true, T(0));
+        xch_load(w[2], word(2 * N + gx), true, T(0));
+        bool ok = xch_take(w[0], f0, n, true);
+        ok &= xch_take(w[1], f1, n, true);
+        ok &= xch_take(w[2], f2, n, true);
+        if (fl & (kXE | kYE | kXH | kYH)) {
+          xch_load(w[0], word(pxe), fl & kXE, T(0));
+          xch_load(w[1], word(pye), fl & kYE, T(0));
+          xch_load(w[2], word(pxh), fl & kXH, T(0));
+          xch_load(w[3], word(pyh), fl & kYH, T(0));
+          ok &= xch_take(w[0], xe, n, fl & kXE);
+          ok &= xch_take(w[1], ye, n, fl & kYE);
+          ok &= xch_take(w[2], xh, n, fl & kXH);
+          ok &= xch_take(w[3], yh, n, fl & kYH);
+        }
+        if (ok || !waits) break;
+        if (clock64() - t0 > p.wait_cycles) {
+          atomicExch(p.state + 1, 3);  // reported to the host by oidt_job_sync
+          waits = false;
+        } else if (++round % 64 == 0 && ld_acquire(p.state + 1) != 0) {  // an earlier wait expired: stop waiting
+          waits = false;
+        }
       }
+      F0[t] = f0;
+      F1[t] = f1;
+      F2[t] = f2;
     }
+    __syncthreads();
   }
+  // ---- owned cells to the other buffer ----------------------------------------------------
+  if (fl & kOwn) {
+    p.fn[FA][g] = f0;
+    p.fn[FB][g] = f1;
+    p.fn[FC][g] = f2;
+    if (fl & kXE) p.psin[EXS][AX][sides & 1][oxE] = xe;
+    if (fl & kYE) p.psin[EYS][AY][(sides >> 1) & 1][oyE] = ye;
+    if (fl & kXH) p.psin[HXS][AX][(sides >> 2) & 1][oxH] = xh;
+    if (fl & kYH) p.psin[HYS][AY][(sides >> 3) & 1][oyH] = yh;
+  }
+  if (nsub > 1 && t == 0) a.epoch[blockIdx.x] = e0 + nsub;
 }
 
 }  // namespace oidt
