@@ -269,7 +269,8 @@ __device__ __forceinline__ void capture(const Params<T> &p, int s, int port, int
 // the read-only path otherwise.
 template <bool CG, typename T> __device__ __forceinline__ T ld_e(const T *q) { return CG ? __ldcg(q) : __ldg(q); }
 
-template <typename T, bool CG = false> struct GlobalAcc3 {
+// IDX: dt/eps from the material index where the job has one.
+template <typename T, bool CG = false, bool IDX = false> struct GlobalAcc3 {
   const Params<T> &p;
   long long c, sy, sx;
   __device__ __forceinline__ T h(int f, int di, int dj, int dk) const { return p.f[f][c + di * sx + dj * sy + dk]; }
@@ -278,7 +279,7 @@ template <typename T, bool CG = false> struct GlobalAcc3 {
   }
   __device__ __forceinline__ T eold(int f) const { return p.f[f][c]; }
   __device__ __forceinline__ T hold(int f) const { return p.f[f][c]; }
-  __device__ __forceinline__ T cb(int a) const { return p.cb[a][c]; }
+  __device__ __forceinline__ T cb(int a) const { return IDX && p.mat ? p.mtab[4 * (int)p.mat[c] + a] : p.cb[a][c]; }
 };
 
 // New E at cell (i, j, k) -> out[EX..EZ] (old value where a component is not
@@ -482,11 +483,11 @@ __device__ __forceinline__ void y3_capture_h(const Params<T> &p, int s, int i, i
 }
 
 // Per-cell launches (in place): E half then H half.
-template <typename T, bool EXACT>
+template <typename T, bool EXACT, bool IDX = false>
 __device__ __forceinline__ void y3_e_cell(const Params<T> &p, int i, int j, int k, int n, int s) {
   const long long sy = p.nzp, sx = (long long)p.ny * p.nzp;
   const long long c = i * sx + j * sy + k;
-  GlobalAcc3<T> a{p, c, sy, sx};
+  GlobalAcc3<T, false, IDX> a{p, c, sy, sx};
   T e[3];
   const int m = y3_e_compute<T, EXACT>(p, a, i, j, k, n, true, e);
   if (m & 1) p.f[EX][c] = e[0];

@@ -44,7 +44,7 @@ constexpr int kVecThreads = 128;
 // blocks (64 registers) spill more and lose (76.1).
 // FP64 with two cells a thread: 97 x 114 x 187 fast 63.9 us per step with
 // seven / six blocks, 64.9 with six / six, 66.7 with six / five; EXACT 107.3,
-// 103.8, 101.7.
+// 103.8, 101.7 (99.4 with v3_src_e out of line).
 template <typename T, bool EXACT> constexpr int kVecBlocksPerSM = sizeof(T) == 8 && EXACT ? 5 : 6;   // H half-step
 template <typename T, bool EXACT> constexpr int kVecBlocksPerSME = sizeof(T) == 8 && EXACT ? 6 : 7;  // E half-step
 
@@ -176,7 +176,7 @@ __device__ __forceinline__ void psi_prefetch(const Params<T> &p, int i, int j, i
 // `yin`) and one branch for all of them, so that their chains overlap.
 // Measured on a B200, 97 x 114 x 187 float64 EXACT: 144 us per step with a
 // test and a branch a quotient, 117 with one a cell, 120 with one a group of
-// four cells, 102 with one a group of two (and six / five blocks an SM);
+// four cells, 102 with one a group of two (and six / five blocks an SM; 99 now);
 // float32 EXACT 88, 84 and 64.
 template <typename T, bool EXACT> __device__ __forceinline__ bool yin3(T y) {
   if constexpr (EXACT) return Ar<T, EXACT>::yin(y);
@@ -258,13 +258,21 @@ __device__ __forceinline__ bool edge_group(const Params<T> &p, const VecGeom &g,
   return true;
 }
 
+// A group's cells next to the source box, E half-step, per cell.  Not inlined:
+// few groups take it, and inlined it costs the others registers (float32 128 x
+// 128 x 256 67.1 -> 66.7 us per step, 48 x 40 x 96 10.6 -> 10.4; float64 EXACT 97
+// x 114 x 187 102.7 -> 99.4).
+template <typename T, bool EXACT>
+__device__ __noinline__ void v3_src_e(const Params<T> &p, int i, int j, int k0, int k1, int s) {
+  for (int k = k0; k < k1; ++k) y3_e_cell<T, EXACT, true>(p, i, j, k, p.state[0] + s, s);
+}
+
 template <typename T, bool EXACT, int W>
 __device__ __forceinline__ void v3_edge_e(const Params<T> &p, const VecGeom &g, int i, int bx, int s) {
   int j, k0;
   if (!edge_group<W>(p, g, bx, j, k0)) return;
   if (near_src(p, i, j, k0, W)) {
-    for (int m = 0; m < W; ++m)
-      if (k0 + m < p.nz) y3_e_cell<T, EXACT>(p, i, j, k0 + m, p.state[0] + s, s);
+    v3_src_e<T, EXACT>(p, i, j, k0, min(k0 + W, p.nz), s);
     return;
   }
   using A = Ar<T, EXACT>;
@@ -742,7 +750,7 @@ __device__ __forceinline__ void v3_e_block(const Params<T> &p, const VecGeom &g,
   const int r = t / g.nvc;
   const int j = p.jb + r, k0 = g.kz0 + W * (t - r * g.nvc);
   if (near_src(p, i, j, k0, W) && p.src_field == HY) {
-    for (int m = 0; m < W; ++m) y3_e_cell<T, EXACT>(p, i, j, k0 + m, p.state[0] + s, s);
+    v3_src_e<T, EXACT>(p, i, j, k0, k0 + W, s);
     return;
   }
   using A = Ar<T, EXACT>;
@@ -1051,7 +1059,7 @@ __device__ __forceinline__ void v3_h_block(const Params<T> &p, const VecGeom &g,
 }
 
 template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kVecThreads, kVecBlocksPerSME<T, EXACT>) k_v3_e(Params<T> p, VecGeom g, int s) {
+__global__ void __launch_bounds__(kVecThreads, kVecBlocksPerSME<T, EXACT>) k_v3_e(const __grid_constant__ Params<T> p, VecGeom g, int s) {
   pdl_wait();
   v3_e_block<T, EXACT, kVecW<T>>(p, g, p.ib + blockIdx.y, blockIdx.x, s);
 }
