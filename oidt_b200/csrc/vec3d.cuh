@@ -24,8 +24,8 @@
 // EXACT arithmetic every operation is the reference's IEEE operation, so
 // float64 runs equal the reference and the oracle bit for bit.
 //
-// Cells next to the source box take the general per-cell path (y3_e_cell /
-// y3_h_cell) in both roles of the E half-step: with the 'TM' source (Hy) the
+// Groups at the source box with cells in an x or z slab take the general
+// per-cell path (y3_e_cell) in both roles of the E half-step: with the 'TM' source (Hy) the
 // reference subtracts J from Hy between the E curl and the E CPML kernels, so
 // the x-slab term of Ez and the z-slab term of Ex read Hy - J there.
 #pragma once
@@ -234,11 +234,28 @@ struct VecGeom {
   int nb_vec;    // blocks of the vector role per plane (the edge role follows)
 };
 
-// One cell within one cell of the source box (widened below in i and k: the
-// E CPML of Ex and Ez reads the Hy source at k + 1 and i + 1).
-template <typename T> __device__ __forceinline__ bool near_src(const Params<T> &p, int i, int j, int k0, int nk) {
-  return p.src_field >= 0 && i >= p.slo[0] - 1 && i < p.shi[0] && j >= p.slo[1] && j < p.shi[1] &&
-         k0 + nk > p.slo[2] - 1 && k0 < p.shi[2];
+// A group whose E CPML terms read the Hy source (the box widened below in i
+// and k: Ez's x-slab term reads Hy at i + 1, Ex's z-slab term at k + 1), in the
+// x slab or (zs: z-slab cells in [k0, k0 + nk)) the z slab.  These run per cell.
+// The other groups at the source do not: all of them in the edge role, and all
+// with a 'TM' source, ran one cell after another, and a half-step of a small
+// grid waited for that chain (float32, source 3 cells from the slab: 64 x 64 x
+// 128 20.8 -> 14.7 us per step; 'TM' 48 x 40 x 96 12.0 -> 10.3).
+template <typename T> __device__ __forceinline__ bool src_in_cpml(const Params<T> &p, int i, int j, int k0, int nk, bool zs) {
+  if (p.src_field != HY || i < p.slo[0] - 1 || i >= p.shi[0] || j < p.slo[1] || j >= p.shi[1] || k0 + nk <= p.slo[2] - 1 ||
+      k0 >= p.shi[2])
+    return false;
+  int d, side;
+  if (e_slab(i, p.ib, p.ie, p.P, d, side) >= 0) return true;
+  if (zs)
+    for (int k = k0; k < k0 + nk; ++k)
+      if (e_slab(k, p.kb, p.ke, p.P, d, side) >= 0) return true;
+  return false;
+}
+// The source box holds cells of the group (field fld).
+template <typename T> __device__ __forceinline__ bool src_group(const Params<T> &p, int fld, int i, int j, int k0, int nk) {
+  return p.src_field == fld && i >= p.slo[0] && i < p.shi[0] && j >= p.slo[1] && j < p.shi[1] && k0 + nk > p.slo[2] &&
+         k0 < p.shi[2];
 }
 
 // Edge role: groups k0 in [0, kz0) and [kz1, nzp) -- the z slabs,
@@ -246,7 +263,7 @@ template <typename T> __device__ __forceinline__ bool near_src(const Params<T> &
 // tested per cell.  A group's z-slab psi values are one 16-byte vector of the
 // padded z-slab rows, unless the group holds cells of both z slabs (then cell
 // by cell); all old values of a group are read before the first write.
-// Groups within one cell of the source box run y3_e_cell / y3_h_cell per cell.
+// Groups of src_in_cpml run y3_e_cell per cell.
 template <int W, typename T>
 __device__ __forceinline__ bool edge_group(const Params<T> &p, const VecGeom &g, int bx, int &j, int &k0) {
   const int nge = g.nedge >> (W == 4 ? 2 : 1);
@@ -258,7 +275,7 @@ __device__ __forceinline__ bool edge_group(const Params<T> &p, const VecGeom &g,
   return true;
 }
 
-// A group's cells next to the source box, E half-step, per cell.  Not inlined:
+// A group's cells per cell, E half-step (src_in_cpml).  Not inlined:
 // few groups take it, and inlined it costs the others registers (float32 128 x
 // 128 x 256 67.1 -> 66.7 us per step, 48 x 40 x 96 10.6 -> 10.4; float64 EXACT 97
 // x 114 x 187 102.7 -> 99.4).
@@ -271,7 +288,7 @@ template <typename T, bool EXACT, int W>
 __device__ __forceinline__ void v3_edge_e(const Params<T> &p, const VecGeom &g, int i, int bx, int s) {
   int j, k0;
   if (!edge_group<W>(p, g, bx, j, k0)) return;
-  if (near_src(p, i, j, k0, W)) {
+  if (src_in_cpml(p, i, j, k0, W, true)) {
     v3_src_e<T, EXACT>(p, i, j, k0, min(k0 + W, p.nz), s);
     return;
   }
@@ -342,6 +359,12 @@ __device__ __forceinline__ void v3_edge_e(const Params<T> &p, const VecGeom &g, 
                     in3<T, EXACT>(dxy);
     if (ok) curl([](T a, T b, T y) { return A::quo(a, b, y); });
     else curl([](T a, T b, T) { return A::ieee(a, b); });
+  }
+  if (src_group(p, EY, i, j, k0, W)) {  // soft source on Ey ('TE'): after the curl, before the CPML terms
+    const T Jn = p.jsrc[p.state[0] + s];
+#pragma unroll
+    for (int m = 0; m < W; ++m)
+      if (mey[m] && k0 + m >= p.slo[2] && k0 + m < p.shi[2]) e1[m] = A::sub(e1[m], Jn);
   }
   int d, side, q;
   if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {  // update_pml_ey_xinc, update_pml_ez_xinc
@@ -501,11 +524,6 @@ template <typename T, bool EXACT, bool CG, int W>
 __device__ __forceinline__ void v3_edge_h(const Params<T> &p, const VecGeom &g, int i, int bx, int s) {
   int j, k0;
   if (!edge_group<W>(p, g, bx, j, k0)) return;
-  if (near_src(p, i, j, k0, W)) {
-    for (int m = 0; m < W; ++m)
-      if (k0 + m < p.nz) y3_h_cell<T, EXACT, CG>(p, i, j, k0 + m, p.state[0] + s, s);
-    return;
-  }
   using A = Ar<T, EXACT>;
   const int P = p.P;
   const bool ihy = i > p.ib, jhx = j > p.jb;
@@ -537,6 +555,12 @@ __device__ __forceinline__ void v3_edge_h(const Params<T> &p, const VecGeom &g, 
   ldw4(Hx, hx + o);
   ldw4(Hy, hy + o);
   ldw4(Hz, hz + o);
+  if (src_group(p, HY, i, j, k0, W)) {  // soft source on Hy ('TM'): subtracted before the Hy update
+    const T Jn = p.jsrc[p.state[0] + s];
+#pragma unroll
+    for (int m = 0; m < W; ++m)
+      if (mhy[m] && k0 + m >= p.slo[2] && k0 + m < p.shi[2]) Hy.v[m] = A::sub(Hy.v[m], Jn);
+  }
   ld4(Rz, p.rkd[5] + k0);
   if (EXACT) ld4(Kz, p.kd[5] + k0);
   const T rkx = p.rkd[3][i], rky = p.rkd[4][j];
@@ -749,7 +773,7 @@ __device__ __forceinline__ void v3_e_block(const Params<T> &p, const VecGeom &g,
   if (t >= (p.je - p.jb) * g.nvc) return;
   const int r = t / g.nvc;
   const int j = p.jb + r, k0 = g.kz0 + W * (t - r * g.nvc);
-  if (near_src(p, i, j, k0, W) && p.src_field == HY) {
+  if (src_in_cpml(p, i, j, k0, W, false)) {
     v3_src_e<T, EXACT>(p, i, j, k0, k0 + W, s);
     return;
   }
@@ -812,8 +836,7 @@ __device__ __forceinline__ void v3_e_block(const Params<T> &p, const VecGeom &g,
     else curl([](T a, T b, T) { return A::ieee(a, b); });
   }
   // soft source on Ey ('TE'): after the curl, before the CPML terms
-  if (p.src_field == EY && mey && i >= p.slo[0] && i < p.shi[0] && j >= p.slo[1] && j < p.shi[1] &&
-      k0 + W > p.slo[2] && k0 < p.shi[2]) {
+  if (mey && src_group(p, EY, i, j, k0, W)) {
     const T Jn = p.jsrc[p.state[0] + s];
 #pragma unroll
     for (int m = 0; m < W; ++m)
@@ -941,8 +964,7 @@ __device__ __forceinline__ void v3_h_block(const Params<T> &p, const VecGeom &g,
   // Hy i = ib, Hz both
   const bool mhx = j > p.jb, mhy = i > p.ib, mhz = mhx && mhy;
   // soft source on Hy ('TM'): subtracted before the Hy update
-  const bool src = p.src_field == HY && mhy && i >= p.slo[0] && i < p.shi[0] && j >= p.slo[1] && j < p.shi[1] &&
-                   k0 + W > p.slo[2] && k0 < p.shi[2];
+  const bool src = mhy && src_group(p, HY, i, j, k0, W);
   const T Jn = src ? p.jsrc[p.state[0] + s] : T(0);
   T h0[W], h1[W], h2[W], dyz[W], dzy[W], dzx[W], dxz[W], dxy[W], dyx[W];
 #pragma unroll
