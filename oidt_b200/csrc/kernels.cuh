@@ -270,13 +270,11 @@ __device__ __forceinline__ void capture(const Params<T> &p, int s, int port, int
 template <bool CG, typename T> __device__ __forceinline__ T ld_e(const T *q) { return CG ? __ldcg(q) : __ldg(q); }
 
 // IDX: dt/eps from the material index where the job has one.
-template <typename T, bool CG = false, bool IDX = false> struct GlobalAcc3 {
+template <typename T, bool IDX = false> struct GlobalAcc3 {
   const Params<T> &p;
   long long c, sy, sx;
   __device__ __forceinline__ T h(int f, int di, int dj, int dk) const { return p.f[f][c + di * sx + dj * sy + dk]; }
-  __device__ __forceinline__ T e(int f, int di, int dj, int dk) const {
-    return CG ? __ldcg(p.f[f] + (c + di * sx + dj * sy + dk)) : p.f[f][c + di * sx + dj * sy + dk];
-  }
+  __device__ __forceinline__ T e(int f, int di, int dj, int dk) const { return p.f[f][c + di * sx + dj * sy + dk]; }
   __device__ __forceinline__ T eold(int f) const { return p.f[f][c]; }
   __device__ __forceinline__ T hold(int f) const { return p.f[f][c]; }
   __device__ __forceinline__ T cb(int a) const { return IDX && p.mat ? p.mtab[4 * (int)p.mat[c] + a] : p.cb[a][c]; }
@@ -487,7 +485,7 @@ template <typename T, bool EXACT, bool IDX = false>
 __device__ __forceinline__ void y3_e_cell(const Params<T> &p, int i, int j, int k, int n, int s) {
   const long long sy = p.nzp, sx = (long long)p.ny * p.nzp;
   const long long c = i * sx + j * sy + k;
-  GlobalAcc3<T, false, IDX> a{p, c, sy, sx};
+  GlobalAcc3<T, IDX> a{p, c, sy, sx};
   T e[3];
   const int m = y3_e_compute<T, EXACT>(p, a, i, j, k, n, true, e);
   if (m & 1) p.f[EX][c] = e[0];
@@ -496,11 +494,11 @@ __device__ __forceinline__ void y3_e_cell(const Params<T> &p, int i, int j, int 
   y3_capture_e(p, s, i, j, k, m, e);
 }
 
-template <typename T, bool EXACT, bool CG = false>
+template <typename T, bool EXACT>
 __device__ __forceinline__ void y3_h_cell(const Params<T> &p, int i, int j, int k, int n, int s) {
   const long long sy = p.nzp, sx = (long long)p.ny * p.nzp;
   const long long c = i * sx + j * sy + k;
-  GlobalAcc3<T, CG> a{p, c, sy, sx};
+  GlobalAcc3<T> a{p, c, sy, sx};
   T h[3];
   const int m = y3_h_compute<T, EXACT>(p, a, i, j, k, n, h);
   if (m & 1) p.f[HX][c] = h[0];

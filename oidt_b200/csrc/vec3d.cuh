@@ -240,7 +240,8 @@ struct VecGeom {
 // The other groups at the source do not: all of them in the edge role, and all
 // with a 'TM' source, ran one cell after another, and a half-step of a small
 // grid waited for that chain (float32, source 3 cells from the slab: 64 x 64 x
-// 128 20.8 -> 14.7 us per step; 'TM' 48 x 40 x 96 12.0 -> 10.3).
+// 128 20.7 -> 14.7 us per step; 'TM' 48 x 40 x 96 12.0 -> 10.2; a 'TM' source in
+// one group with z-slab cells, 3 cells away at most, 20.4 -> 22.9).
 template <typename T> __device__ __forceinline__ bool src_in_cpml(const Params<T> &p, int i, int j, int k0, int nk, bool zs) {
   if (p.src_field != HY || i < p.slo[0] - 1 || i >= p.shi[0] || j < p.slo[1] || j >= p.shi[1] || k0 + nk <= p.slo[2] - 1 ||
       k0 >= p.shi[2])
