@@ -1,0 +1,44 @@
+"""The vector form's step kernels read their parameter block (about 1 KB) from
+kernel parameter space.  A block passed by value, and then by reference to a
+function that is not inlined, is first copied into each thread's local memory:
+the kernel's stack frame is then larger than the block.  Without the copy a
+frame holds spills only (at most 80 bytes a thread as these kernels compile),
+so half a block separates the two.  nvcc cross-compiles: no GPU."""
+import os
+import re
+import shutil
+import subprocess
+
+import pytest
+
+from oidt_b200.build import FLAGS, HERE, NVCC, ROOT
+
+SRC = """
+#include "oidt.h"
+#include "kernels.cuh"
+#include "vec3d.cuh"
+using namespace oidt;
+template <typename T, bool X> void *e() { return (void *)k_v3_e<T, X>; }
+template <typename T, bool X> void *h() { return (void *)k_v3_h<T, X>; }
+template <typename T, bool X> void *w() { return (void *)k_v3_wave<T, X>; }
+template <typename T, bool X> struct Forms { void *f[3] = {e<T, X>(), h<T, X>(), w<T, X>()}; };
+Forms<float, false> ff;
+Forms<float, true> fx;
+Forms<double, false> df;
+Forms<double, true> dx;
+static_assert(sizeof(Params<float>) >= 512 && sizeof(Params<double>) >= 512, "a frame below 512 bytes holds no copy");
+"""
+
+
+@pytest.mark.skipif(not (os.path.exists(NVCC) or shutil.which(NVCC)), reason="needs nvcc")
+def test_step_kernels_hold_no_copy_of_their_parameters(tmp_path):
+    src = tmp_path / "frames.cu"
+    src.write_text(SRC)
+    flags = [f for f in FLAGS if f not in ("-shared", "-lineinfo")]
+    r = subprocess.run([NVCC] + flags + ["-Xptxas=-v", "-cubin", "-I", os.path.join(HERE, "csrc"), "-I",
+                                         os.path.join(ROOT, "include"), "-o", str(tmp_path / "frames.cubin"), str(src)],
+                       capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    frames = dict(re.findall(r"Function properties for (\w*k_v3_\w+)\s+(\d+) bytes stack frame", r.stderr))
+    assert len(frames) == 12, r.stderr
+    assert {k: v for k, v in frames.items() if int(v) >= 512} == {}
