@@ -1038,13 +1038,28 @@ template <typename T> VecGeom vec_geom(const Params<T> &p, int W) {
   return vec_geom_of(p.kb, p.ke, p.P, p.jb, p.je, p.nzp, W);
 }
 
+// Whether E CPML terms of a job read its 'TM' source (Hy): an x-slab cell has
+// the box at i or i + 1, or a z-slab cell at k or k + 1.  Such jobs' E
+// half-steps are instances of their own (vec3d.cuh, src_diffs).
+template <typename T> bool src_meets_cpml(const Params<T> &p) {
+  if (p.src_field != HY) return false;
+  for (int a = 0; a < 3; ++a)
+    if (p.slo[a] >= p.shi[a]) return false;
+  auto meets = [&](int a, int b, int e) {  // [slo - 1, shi) and a slab
+    const int lo = p.slo[a] - 1, hi = p.shi[a];
+    return (lo < b + p.P && hi > b) || (lo < e && hi > e - p.P);
+  };
+  return meets(0, p.ib, p.ie) || meets(2, p.kb, p.ke);
+}
+
 // One 3D vector-form half-step: the vector-role blocks, then the edge-role
 // blocks, of one x-plane per grid row.
 template <typename T, bool EXACT> void v3_half(bool H, bool pdl, const Params<T> &p, int s, cudaStream_t st) {
   const VecGeom g = vec_geom(p, kVecW<T>);
   const long long nb_edge = vec_edge_blocks(g, p.jb, p.je, kVecW<T>);
   const dim3 grd((unsigned)(g.nb_vec + nb_edge), p.ie - p.ib), blk(kVecThreads);
-  void (*kern)(const Params<T>, VecGeom, int) = H ? k_v3_h<T, EXACT> : k_v3_e<T, EXACT>;
+  void (*kern)(const Params<T>, VecGeom, int) =
+      H ? k_v3_h<T, EXACT> : src_meets_cpml(p) ? k_v3_e<T, EXACT, true> : k_v3_e<T, EXACT, kSrcCells<T, EXACT>>;
   if (pdl) launch_step_kernel(kern, grd, blk, 0, st, p, g, s);
   else kern<<<grd, blk, 0, st>>>(p, g, s);
 }
@@ -1066,8 +1081,10 @@ template <typename T, bool EXACT> void v3_wave(Job *J, bool pdl, const Params<T>
   w.nb = g.nb_vec + vec_edge_blocks(g, p.jb, p.je, 4);
   w.lag = wave_lag(p);
   const dim3 grd((unsigned)(2LL * (p.ie - p.ib) * w.nb)), blk(kVecThreads);
-  if (pdl) launch_step_kernel(k_v3_wave<T, EXACT>, grd, blk, 0, st, p, g, w, s);
-  else k_v3_wave<T, EXACT><<<grd, blk, 0, st>>>(p, g, w, s);
+  void (*kern)(const Params<T>, VecGeom, WaveArgs, int) =
+      src_meets_cpml(p) ? k_v3_wave<T, EXACT, true> : k_v3_wave<T, EXACT, kSrcCells<T, EXACT>>;
+  if (pdl) launch_step_kernel(kern, grd, blk, 0, st, p, g, w, s);
+  else kern<<<grd, blk, 0, st>>>(p, g, w, s);
 }
 
 // A launch of the tile form's kernel: cooperative (several sub-blocks), or

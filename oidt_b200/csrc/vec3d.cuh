@@ -24,10 +24,9 @@
 // EXACT arithmetic every operation is the reference's IEEE operation, so
 // float64 runs equal the reference and the oracle bit for bit.
 //
-// Groups at the source box with cells in an x or z slab take the general
-// per-cell path (y3_e_cell) in both roles of the E half-step: with the 'TM' source (Hy) the
-// reference subtracts J from Hy between the E curl and the E CPML kernels, so
-// the x-slab term of Ez and the z-slab term of Ex read Hy - J there.
+// With the 'TM' source (Hy) the reference subtracts J from Hy between the E
+// curl and the E CPML kernels, so the x-slab term of Ez and the z-slab term of
+// Ex read Hy - J (src_diffs).
 #pragma once
 #include "kernels.cuh"
 
@@ -234,25 +233,59 @@ struct VecGeom {
   int nb_vec;    // blocks of the vector role per plane (the edge role follows)
 };
 
-// A group whose E CPML terms read the Hy source (the box widened below in i
-// and k: Ez's x-slab term reads Hy at i + 1, Ex's z-slab term at k + 1), in the
-// x slab or (zs: z-slab cells in [k0, k0 + nk)) the z slab.  These run per cell.
-// The other groups at the source do not: all of them in the edge role, and all
-// with a 'TM' source, ran one cell after another, and a half-step of a small
-// grid waited for that chain (float32, source 3 cells from the slab: 64 x 64 x
-// 128 20.7 -> 14.7 us per step; 'TM' 48 x 40 x 96 12.0 -> 10.2; a 'TM' source in
-// one group with z-slab cells, 3 cells away at most, 20.4 -> 22.9).
+// 'TM' source (Hy): Ez's x-slab term reads Hy - J at i and i + 1, Ex's z-slab
+// term at k and k + 1.  Only the E half-steps of jobs whose source meets a slab
+// so (SRC; engine.cu, src_meets_cpml) hold anything for it: in every job's it
+// takes registers (float32 128 x 128 x 256 64.5 us per step without, 65.4 with).
+//
+// src_diffs forms the differences of a group's x- and z-slab terms again, with
+// Hy - J at the cells of the source box.  Measured on a B200, float32, 'TM'
+// source in, at or 2 cells past the z slab, against the group's cells one after
+// another inline / out of line: 48 x 40 x 96 10.2 against 20.4 / 21.3 us per
+// step, 64 x 64 x 128 14.8 against 20.8-23.0 / 23.3-24.8, 128 x 128 x 256 65.4
+// against 67.3 / 68.1.
+template <typename T, bool EXACT, int W>
+__device__ __forceinline__ void src_diffs(const Params<T> &p, int i, int j, int k0, int s, const T (&hy)[W], T hyk,
+                                          const T (&hyx)[W], T (&dyz)[W], T (&dyx)[W]) {
+  using A = Ar<T, EXACT>;
+  if (p.src_field != HY || i < p.slo[0] - 1 || i >= p.shi[0] || j < p.slo[1] || j >= p.shi[1] || k0 + W < p.slo[2] ||
+      k0 >= p.shi[2])
+    return;
+  const T Jn = p.jsrc[p.state[0] + s];
+  const bool in0 = i >= p.slo[0], in1 = i + 1 < p.shi[0];  // the box holds cells of plane i, of plane i + 1
+#pragma unroll
+  for (int m = 0; m < W; ++m) {
+    const int k = k0 + m;
+    const bool at = k >= p.slo[2] && k < p.shi[2], next = k + 1 >= p.slo[2] && k + 1 < p.shi[2];
+    const T h1 = m < W - 1 ? hy[m < W - 1 ? m + 1 : 0] : hyk;
+    const T c = in0 && at ? A::sub(hy[m], Jn) : hy[m];
+    dyz[m] = A::sub(in0 && next ? A::sub(h1, Jn) : h1, c);
+    dyx[m] = A::sub(in1 && at ? A::sub(hyx[m], Jn) : hyx[m], c);
+  }
+}
+// float32 EXACT: such groups run cell after cell, out of line (v3_src_e), and
+// every job's kernel holds the call: without it, or with src_diffs, the code
+// the compiler makes of the EXACT branches is slower (128 x 128 x 256 195 -> 226
+// us per step while most of the grid is still below the fast quotient's range,
+// 99 -> 101 over a whole run; 72 x 80 x 192 74 -> 87).
+template <typename T, bool EXACT> constexpr bool kSrcCells = sizeof(T) == 4 && EXACT;
+// A cell of the group has a term that reads the source (zs: z slabs too).
 template <typename T> __device__ __forceinline__ bool src_in_cpml(const Params<T> &p, int i, int j, int k0, int nk, bool zs) {
-  if (p.src_field != HY || i < p.slo[0] - 1 || i >= p.shi[0] || j < p.slo[1] || j >= p.shi[1] || k0 + nk <= p.slo[2] - 1 ||
+  if (p.src_field != HY || i < p.slo[0] - 1 || i >= p.shi[0] || j < p.slo[1] || j >= p.shi[1] || k0 + nk < p.slo[2] ||
       k0 >= p.shi[2])
     return false;
   int d, side;
-  if (e_slab(i, p.ib, p.ie, p.P, d, side) >= 0) return true;
-  if (zs)
-    for (int k = k0; k < k0 + nk; ++k)
+  if (k0 + nk > p.slo[2] && e_slab(i, p.ib, p.ie, p.P, d, side) >= 0) return true;
+  if (zs && i >= p.slo[0])
+    for (int k = max(k0, p.slo[2] - 1); k < min(k0 + nk, p.shi[2]); ++k)
       if (e_slab(k, p.kb, p.ke, p.P, d, side) >= 0) return true;
   return false;
 }
+template <typename T, bool EXACT>
+__device__ __noinline__ void v3_src_e(const Params<T> &p, int i, int j, int k0, int k1, int s) {
+  for (int k = k0; k < k1; ++k) y3_e_cell<T, EXACT, true>(p, i, j, k, p.state[0] + s, s);
+}
+
 // The source box holds cells of the group (field fld).
 template <typename T> __device__ __forceinline__ bool src_group(const Params<T> &p, int fld, int i, int j, int k0, int nk) {
   return p.src_field == fld && i >= p.slo[0] && i < p.shi[0] && j >= p.slo[1] && j < p.shi[1] && k0 + nk > p.slo[2] &&
@@ -264,7 +297,6 @@ template <typename T> __device__ __forceinline__ bool src_group(const Params<T> 
 // tested per cell.  A group's z-slab psi values are one 16-byte vector of the
 // padded z-slab rows, unless the group holds cells of both z slabs (then cell
 // by cell); all old values of a group are read before the first write.
-// Groups of src_in_cpml run y3_e_cell per cell.
 template <int W, typename T>
 __device__ __forceinline__ bool edge_group(const Params<T> &p, const VecGeom &g, int bx, int &j, int &k0) {
   const int nge = g.nedge >> (W == 4 ? 2 : 1);
@@ -276,23 +308,15 @@ __device__ __forceinline__ bool edge_group(const Params<T> &p, const VecGeom &g,
   return true;
 }
 
-// A group's cells per cell, E half-step (src_in_cpml).  Not inlined:
-// few groups take it, and inlined it costs the others registers (float32 128 x
-// 128 x 256 67.1 -> 66.7 us per step, 48 x 40 x 96 10.6 -> 10.4; float64 EXACT 97
-// x 114 x 187 102.7 -> 99.4).
-template <typename T, bool EXACT>
-__device__ __noinline__ void v3_src_e(const Params<T> &p, int i, int j, int k0, int k1, int s) {
-  for (int k = k0; k < k1; ++k) y3_e_cell<T, EXACT, true>(p, i, j, k, p.state[0] + s, s);
-}
-
-template <typename T, bool EXACT, int W>
+template <typename T, bool EXACT, int W, bool SRC>
 __device__ __forceinline__ void v3_edge_e(const Params<T> &p, const VecGeom &g, int i, int bx, int s) {
   int j, k0;
   if (!edge_group<W>(p, g, bx, j, k0)) return;
-  if (src_in_cpml(p, i, j, k0, W, true)) {
-    v3_src_e<T, EXACT>(p, i, j, k0, min(k0 + W, p.nz), s);
-    return;
-  }
+  if constexpr (SRC && kSrcCells<T, EXACT>)
+    if (src_in_cpml(p, i, j, k0, W, true)) {
+      v3_src_e<T, EXACT>(p, i, j, k0, min(k0 + W, p.nz), s);
+      return;
+    }
   using A = Ar<T, EXACT>;
   const int P = p.P;
   const bool iex = i > p.ib, jey = j > p.jb;
@@ -367,6 +391,7 @@ __device__ __forceinline__ void v3_edge_e(const Params<T> &p, const VecGeom &g, 
     for (int m = 0; m < W; ++m)
       if (mey[m] && k0 + m >= p.slo[2] && k0 + m < p.shi[2]) e1[m] = A::sub(e1[m], Jn);
   }
+  if constexpr (SRC && !kSrcCells<T, EXACT>) src_diffs<T, EXACT, W>(p, i, j, k0, s, Hy.v, hyk, Hyx.v, dyz, dyx);
   int d, side, q;
   if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {  // update_pml_ey_xinc, update_pml_ez_xinc
     const long long oa = ((long long)d * p.ny + j) * p.psx + k0;
@@ -764,20 +789,21 @@ __device__ __forceinline__ void v3_edge_h(const Params<T> &p, const VecGeom &g, 
 // then edge-role blocks, x-planes ib..ie-1).
 // ---------------------------------------------------------------------------
 // One block of x-plane i: bx < nb_vec a vector-role block, the edge role above.
-template <typename T, bool EXACT, int W>
+template <typename T, bool EXACT, int W, bool SRC>
 __device__ __forceinline__ void v3_e_block(const Params<T> &p, const VecGeom &g, int i, int bx, int s) {
   if (bx >= g.nb_vec) {
-    v3_edge_e<T, EXACT, W>(p, g, i, bx, s);
+    v3_edge_e<T, EXACT, W, SRC>(p, g, i, bx, s);
     return;
   }
   const int t = bx * kVecThreads + threadIdx.x;
   if (t >= (p.je - p.jb) * g.nvc) return;
   const int r = t / g.nvc;
   const int j = p.jb + r, k0 = g.kz0 + W * (t - r * g.nvc);
-  if (src_in_cpml(p, i, j, k0, W, false)) {
-    v3_src_e<T, EXACT>(p, i, j, k0, k0 + W, s);
-    return;
-  }
+  if constexpr (SRC && kSrcCells<T, EXACT>)
+    if (src_in_cpml(p, i, j, k0, W, false)) {
+      v3_src_e<T, EXACT>(p, i, j, k0, k0 + W, s);
+      return;
+    }
   using A = Ar<T, EXACT>;
   const int sy = p.nzp;
   const long long sx = (long long)p.ny * p.nzp, bi = (long long)i * sx;
@@ -843,6 +869,7 @@ __device__ __forceinline__ void v3_e_block(const Params<T> &p, const VecGeom &g,
     for (int m = 0; m < W; ++m)
       if (k0 + m >= p.slo[2] && k0 + m < p.shi[2]) e1[m] = A::sub(e1[m], Jn);
   }
+  if constexpr (SRC && !kSrcCells<T, EXACT>) src_diffs<T, EXACT, W>(p, i, j, k0, s, Hy.v, hyk, Hyx.v, dyz, dyx);
   const int P = p.P;
   int d, side, q;
   if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {  // update_pml_ey_xinc, update_pml_ez_xinc
@@ -1081,10 +1108,10 @@ __device__ __forceinline__ void v3_h_block(const Params<T> &p, const VecGeom &g,
   }
 }
 
-template <typename T, bool EXACT>
+template <typename T, bool EXACT, bool SRC>
 __global__ void __launch_bounds__(kVecThreads, kVecBlocksPerSME<T, EXACT>) k_v3_e(const __grid_constant__ Params<T> p, VecGeom g, int s) {
   pdl_wait();
-  v3_e_block<T, EXACT, kVecW<T>>(p, g, p.ib + blockIdx.y, blockIdx.x, s);
+  v3_e_block<T, EXACT, kVecW<T>, SRC>(p, g, p.ib + blockIdx.y, blockIdx.x, s);
 }
 
 template <typename T, bool EXACT>
@@ -1121,8 +1148,8 @@ struct WaveArgs {
 
 // __grid_constant__, as in k_v3_e: v3_src_e takes the parameters by reference,
 // and of a plain by-value parameter each thread would keep a copy of 1 KB in
-// local memory (128 x 128 x 256 float32 393 us per step with it, 83 without).
-template <typename T, bool EXACT>
+// local memory (128 x 128 x 256 float32 393 us per step with it, 82 without).
+template <typename T, bool EXACT, bool SRC>
 __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? kVecBlocksPerSM<T, EXACT> : 3)
     k_v3_wave(const __grid_constant__ Params<T> p, VecGeom g, WaveArgs w, int s) {
   pdl_wait();
@@ -1143,7 +1170,7 @@ __global__ void __launch_bounds__(kVecThreads, sizeof(T) == 4 ? kVecBlocksPerSM<
     q = n - D + (u - D - 2 * (n - D));
   }
   if (!is_h) {
-    v3_e_block<T, EXACT, 4>(p, g, p.ib + q, bx, s);
+    v3_e_block<T, EXACT, 4, SRC>(p, g, p.ib + q, bx, s);
     __threadfence();  // this thread's stores visible to the whole GPU ...
     __syncthreads();  // ... for every thread of the block, before the count
     if (threadIdx.x == 0) atomicAdd(w.done + q, 1);

@@ -2,7 +2,7 @@
 kernel parameter space.  A block passed by value, and then by reference to a
 function that is not inlined, is first copied into each thread's local memory:
 the kernel's stack frame is then larger than the block.  Without the copy a
-frame holds spills only (at most 80 bytes a thread as these kernels compile),
+frame holds spills only (at most 168 bytes a thread as these kernels compile),
 so half a block separates the two.  nvcc cross-compiles: no GPU."""
 import os
 import re
@@ -18,10 +18,12 @@ SRC = """
 #include "kernels.cuh"
 #include "vec3d.cuh"
 using namespace oidt;
-template <typename T, bool X> void *e() { return (void *)k_v3_e<T, X>; }
+template <typename T, bool X, bool S> void *e() { return (void *)k_v3_e<T, X, S>; }
 template <typename T, bool X> void *h() { return (void *)k_v3_h<T, X>; }
-template <typename T, bool X> void *w() { return (void *)k_v3_wave<T, X>; }
-template <typename T, bool X> struct Forms { void *f[3] = {e<T, X>(), h<T, X>(), w<T, X>()}; };
+template <typename T, bool X, bool S> void *w() { return (void *)k_v3_wave<T, X, S>; }
+template <typename T, bool X> struct Forms {  // S: a 'TM' source that the E CPML terms read
+  void *f[5] = {e<T, X, kSrcCells<T, X>>(), e<T, X, true>(), h<T, X>(), w<T, X, kSrcCells<T, X>>(), w<T, X, true>()};
+};
 Forms<float, false> ff;
 Forms<float, true> fx;
 Forms<double, false> df;
@@ -40,5 +42,5 @@ def test_step_kernels_hold_no_copy_of_their_parameters(tmp_path):
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     frames = dict(re.findall(r"Function properties for (\w*k_v3_\w+)\s+(\d+) bytes stack frame", r.stderr))
-    assert len(frames) == 12, r.stderr
+    assert len(frames) == 18, r.stderr  # float32 EXACT has one instance of each for both
     assert {k: v for k, v in frames.items() if int(v) >= 512} == {}
