@@ -41,7 +41,8 @@
 // behind per-tile counters (fence, release, acquire, then the loads) took 3.5 us
 // where the words take 2.1.  Measured on a B200, 400 x 200 float64 in sub-blocks
 // of 4: EXACT 2.95 -> 2.62 us per step with the words, -> 2.45 with the range
-// test on the integer pipe (kernels.cuh, Ar); fast 2.08 -> 1.97.
+// test on the integer pipe (kernels.cuh, Ar), -> 2.30 without spills in the
+// steps; fast 2.09 -> 1.64 with the words and without spills.
 //
 // Per cell the arithmetic is that of kernels.cuh's tm2_e_cell / tm2_h_cell /
 // te2_e_cell / te2_h_cell (the reference's fdtd_funcs.py of FDTD_2D_TM and
@@ -160,16 +161,26 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
   const int nrow = wi1 - wi0, ncol = wj1 - wj0;
   const int t = threadIdx.x;
   const bool act = t < nrow * ncol;
-  const int li = act ? t / ncol : 0, lj = act ? t - li * ncol : 0, i = wi0 + li, j = wj0 + lj;
-  int gx = i * ny + j;
-  const int g = gx;  // the cell in the [nx][ny] arrays (2^31 cells at most)
+  const int li = act ? t / ncol : 0, lj = act ? t - li * ncol : 0;
+  int i = wi0 + li, j = wj0 + lj;
+  auto cell = [&] { return i * ny + j; };  // the cell in the [nx][ny] arrays (2^31 cells at most)
+  // its place in the x-slab [side][P][ny] and y-slab [side][nx][P] psi arrays (an H-slab cell is an E-slab cell
+  // of the same layer and side).  These, the captures' and the exchange words' places are formed where they are
+  // used: held through the steps they took some twenty of a thread's 64 registers, and the float64 kernels
+  // spilled in the steps (64 to 72 bytes a thread; 8 to 16 now).  400 x 200 float64 fast 1.96 -> 1.64 us per
+  // step, EXACT 2.45 -> 2.30; 603 x 1601 (waves) 25.8 -> 22.5 and 30.0 -> 26.8.
+  auto xslab = [&](int &side) {
+    side = i < p.ib + P ? LO : HI;
+    return (side ? i - p.ie + P : i - p.ib) * ny + j;
+  };
+  auto yslab = [&](int &side) {
+    side = j < p.jb + P ? LO : HI;
+    return i * P + (side ? j - p.je + P : j - p.jb);
+  };
   // ---- the cell's constants ------------------------------------------------------------
   unsigned fl = 0;
   int qE = 0, qH = 0;  // slab coefficient indices + 1: x slab in bits 0-15, y slab in bits 16-31
   T cbA = T(0), cbB = T(0);  // dt/eps of the cell's E components
-  int capE[2] = {0, 0}, capH[2] = {0, 0};  // ring offsets of the cell's captures within a slot, per port
-  // psi offsets of the cell in its slab arrays (x slab [P][ny], y slab [nx][P]) and their sides
-  int oxE = 0, oyE = 0, oxH = 0, oyH = 0, sides = 0;  // sides: bit 0 x E, 1 y E, 2 x H, 3 y H
   // this thread's entries of the coefficient and kappa dx tables, loaded first so that
   // their latency overlaps the cell's own loads (leftovers past kTileThreads below)
   const int nk = 4 * (nrow + ncol);
@@ -187,26 +198,18 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
   if (act) {
     int d, side, q;
     if ((q = e_slab(i, p.ib, p.ie, P, d, side)) >= 0) {
-      oxE = d * ny + j;
-      sides |= side;
       fl |= kXE;
       qE |= q + 1;
     }
     if ((q = e_slab(j, p.jb, p.je, P, d, side)) >= 0) {
-      oyE = i * P + d;
-      sides |= side << 1;
       fl |= kYE;
       qE |= (q + 1) << 16;
     }
     if ((q = h_slab(i, p.ib, p.ie, P, d, side)) >= 0) {
-      oxH = d * ny + j;
-      sides |= side << 2;
       fl |= kXH;
       qH |= q + 1;
     }
     if ((q = h_slab(j, p.jb, p.je, P, d, side)) >= 0) {
-      oyH = i * P + d;
-      sides |= side << 3;
       fl |= kYH;
       qH |= (q + 1) << 16;
     }
@@ -221,26 +224,20 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
       if (i >= p.ib && i < p.ie && j > p.jb && j < p.je && left) fl |= kH1;          // update_hx :53-58
       if (i > p.ib && i < p.ie && j >= p.jb && j < p.je && down) fl |= kH2;          // update_hy :62-67
       if (in_src(p, EZ, i, j, 0)) fl |= kSrc;
-      cbA = __ldg(p.cb[2] + g);
+      cbA = __ldg(p.cb[2] + cell());
     } else {
       if (i > p.ib && i < p.ie && j >= p.jb && j < p.je && right) fl |= kE1;         // update_ex :43-49
       if (i >= p.ib && i < p.ie && j > p.jb && j < p.je && up) fl |= kE2;            // update_ey :52-58
       if (i > p.ib && i < p.ie && j > p.jb && j < p.je && down && left) fl |= kH1;   // update_hz :61-67
       if (in_src(p, HZ, i, j, 0)) fl |= kSrc;
-      cbA = __ldg(p.cb[0] + g);
-      cbB = __ldg(p.cb[1] + g);
+      cbA = __ldg(p.cb[0] + cell());
+      cbB = __ldg(p.cb[1] + cell());
     }
     // ring captures of an owned cell on a port plane (where the update of the captured component runs)
     for (int port = 0; port < 2 && own; ++port) {
       const int x = p.port_pos[port];
-      if (i == x && (fl & (TM ? kE1 : kE2))) {
-        fl |= kCE0 << port;
-        capE[port] = (port * p.nslot + 0) * (int)p.plane + j;
-      }
-      if ((i == x || i == x + 1) && (fl & (TM ? kH2 : kH1))) {
-        fl |= kCH0 << port;
-        capH[port] = (port * p.nslot + (i == x ? 1 : 2)) * (int)p.plane + j;
-      }
+      if (i == x && (fl & (TM ? kE1 : kE2))) fl |= kCE0 << port;
+      if ((i == x || i == x + 1) && (fl & (TM ? kH2 : kH1))) fl |= kCH0 << port;
     }
   }
   if (t < 4 * P) BE[t] = vco;  // the CPML coefficients be ce bh ch, and the kappa dx tables
@@ -260,18 +257,30 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
   const int e0 = nsub > 1 ? a.epoch[blockIdx.x] : 0;  // equal for every tile at launch
   T f0 = T(0), f1 = T(0), f2 = T(0), xe = T(0), ye = T(0), xh = T(0), yh = T(0);  // the cell's values
   if (act) {  // the held tile
+    const int g = cell();
     f0 = __ldcg(p.f[FA] + g);
     f1 = __ldcg(p.f[FB] + g);
     f2 = __ldcg(p.f[FC] + g);
     F0[t] = f0;
     F1[t] = f1;
     F2[t] = f2;
-    if (fl & kXE) xe = __ldcg(p.psi[EXS][AX][sides & 1] + oxE);
-    if (fl & kYE) ye = __ldcg(p.psi[EYS][AY][(sides >> 1) & 1] + oyE);
-    if (fl & kXH) xh = __ldcg(p.psi[HXS][AX][(sides >> 2) & 1] + oxH);
-    if (fl & kYH) yh = __ldcg(p.psi[HYS][AY][(sides >> 3) & 1] + oyH);
+    int sx, sy;
+    const int ox = xslab(sx), oy = yslab(sy);
+    if (fl & kXE) xe = __ldcg(p.psi[EXS][AX][sx] + ox);
+    if (fl & kYE) ye = __ldcg(p.psi[EYS][AY][sy] + oy);
+    if (fl & kXH) xh = __ldcg(p.psi[HXS][AX][sx] + ox);
+    if (fl & kYH) yh = __ldcg(p.psi[HYS][AY][sy] + oy);
   }
   __syncthreads();
+  // captures of an owned cell into the step's ring slot: E to slot 0, H to slot 1 (x = port) or 2 (x = port + 1)
+  auto capture_e = [&](T *ring, T v) {
+    if (fl & kCE0) ring[j] = v;
+    if (fl & kCE1) ring[p.nslot * (int)p.plane + j] = v;
+  };
+  auto capture_h = [&](T *ring, T v) {
+    if (fl & kCH0) ring[(i == p.port_pos[0] ? 1 : 2) * (int)p.plane + j] = v;
+    if (fl & kCH1) ring[(p.nslot + (i == p.port_pos[1] ? 1 : 2)) * (int)p.plane + j] = v;
+  };
   bool waits = true;
   for (int sb = 0; sb < nsub; ++sb) {
     const int s1 = min(a.cnt, (sb + 1) * H);
@@ -296,8 +305,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
           }
           f0 = e;
           F0[t] = e;
-          if (fl & kCE0) ring[capE[0]] = e;
-          if (fl & kCE1) ring[capE[1]] = e;
+          if (fl & (kCE0 | kCE1)) capture_e(ring, e);
         }
       } else {
         if (fl & kE1) {  // update_ex :43-49
@@ -321,8 +329,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
           }
           f1 = e;
           F1[t] = e;
-          if (fl & kCE0) ring[capE[0]] = e;
-          if (fl & kCE1) ring[capE[1]] = e;
+          if (fl & (kCE0 | kCE1)) capture_e(ring, e);
         }
       }
       __syncthreads();
@@ -349,8 +356,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
           }
           f2 = h;
           F2[t] = h;
-          if (fl & kCH0) ring[capH[0]] = h;
-          if (fl & kCH1) ring[capH[1]] = h;
+          if (fl & (kCH0 | kCH1)) capture_h(ring, h);
         }
       } else {
         if (fl & kH1) {  // update_hz :61-67
@@ -370,8 +376,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
           }
           f2 = h;
           F2[t] = h;
-          if (fl & kCH0) ring[capH[0]] = h;
-          if (fl & kCH1) ring[capH[1]] = h;
+          if (fl & (kCH0 | kCH1)) capture_h(ring, h);
         }
       }
       __syncthreads();
@@ -379,27 +384,35 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
     if (sb == nsub - 1) break;
     // ---- between sub-blocks: put the owned cells other tiles hold, fetch the halo cells ----
     const unsigned n = (unsigned)(e0 + sb + 1);
-    asm volatile("" : "+r"(gx), "+r"(sides));  // the words' places are formed here, not held through the steps
     constexpr int XW = (int)sizeof(T) / 4;
     const int N = nx * ny, SX = 2 * P * ny, SY = 2 * nx * P;
     unsigned long long *const xb = a.xch + ((n & 1) ? a.xbuf : 0);
     auto word = [&](int v) { return xb + (long long)XW * v; };
-    const int pxe = 3 * N + (sides & 1) * P * ny + oxE, pxh = 3 * N + SX + ((sides >> 2) & 1) * P * ny + oxH;
-    const int pye = 3 * N + 2 * SX + ((sides >> 1) & 1) * nx * P + oyE, pyh = 3 * N + 2 * SX + SY + ((sides >> 3) & 1) * nx * P + oyH;
+    auto places = [&](int &gx, int &pxe, int &pye) {  // of the cell's fields, x-slab and y-slab psi of E (H: + SX, + SY)
+      asm volatile("" : "+r"(i), "+r"(j));  // formed anew at each use
+      int sx, sy;
+      const int ox = xslab(sx), oy = yslab(sy);
+      gx = cell();
+      pxe = 3 * N + sx * P * ny + ox;
+      pye = 3 * N + 2 * SX + sy * nx * P + oy;
+    };
+    int gx, pxe, pye;
     if (fl & kBand) {
+      places(gx, pxe, pye);
       xch_put(word(gx), f0, n);
       xch_put(word(N + gx), f1, n);
       xch_put(word(2 * N + gx), f2, n);
       if (fl & kXE) xch_put(word(pxe), xe, n);
       if (fl & kYE) xch_put(word(pye), ye, n);
-      if (fl & kXH) xch_put(word(pxh), xh, n);
-      if (fl & kYH) xch_put(word(pyh), yh, n);
+      if (fl & kXH) xch_put(word(pxe + SX), xh, n);
+      if (fl & kYH) xch_put(word(pye + SY), yh, n);
     }
     if (act && !(fl & kOwn)) {
       const long long t0 = clock64();
       unsigned round = 0;
       for (;;) {
         unsigned long long w[4][XW] = {};
+        places(gx, pxe, pye);
         xch_load(w[0], word(gx), true, T(0));
         xch_load(w[1], word(N + gx), true, T(0));
         xch_load(w[2], word(2 * N + gx), true, T(0));
@@ -409,8 +422,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
         if (fl & (kXE | kYE | kXH | kYH)) {
           xch_load(w[0], word(pxe), fl & kXE, T(0));
           xch_load(w[1], word(pye), fl & kYE, T(0));
-          xch_load(w[2], word(pxh), fl & kXH, T(0));
-          xch_load(w[3], word(pyh), fl & kYH, T(0));
+          xch_load(w[2], word(pxe + SX), fl & kXH, T(0));
+          xch_load(w[3], word(pye + SY), fl & kYH, T(0));
           ok &= xch_take(w[0], xe, n, fl & kXE);
           ok &= xch_take(w[1], ye, n, fl & kYE);
           ok &= xch_take(w[2], xh, n, fl & kXH);
@@ -432,13 +445,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_2d_tile(const __grid_consta
   }
   // ---- owned cells to the other buffer ----------------------------------------------------
   if (fl & kOwn) {
+    const int g = cell();
     p.fn[FA][g] = f0;
     p.fn[FB][g] = f1;
     p.fn[FC][g] = f2;
-    if (fl & kXE) p.psin[EXS][AX][sides & 1][oxE] = xe;
-    if (fl & kYE) p.psin[EYS][AY][(sides >> 1) & 1][oyE] = ye;
-    if (fl & kXH) p.psin[HXS][AX][(sides >> 2) & 1][oxH] = xh;
-    if (fl & kYH) p.psin[HYS][AY][(sides >> 3) & 1][oyH] = yh;
+    int sx, sy;
+    const int ox = xslab(sx), oy = yslab(sy);
+    if (fl & kXE) p.psin[EXS][AX][sx][ox] = xe;
+    if (fl & kYE) p.psin[EYS][AY][sy][oy] = ye;
+    if (fl & kXH) p.psin[HXS][AX][sx][ox] = xh;
+    if (fl & kYH) p.psin[HYS][AY][sy][oy] = yh;
   }
   if (nsub > 1 && t == 0) a.epoch[blockIdx.x] = e0 + nsub;
 }
