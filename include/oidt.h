@@ -149,7 +149,7 @@ typedef struct oidt_job_desc {
 
 typedef struct oidt_stats {
   uint64_t hbm_budget;   /* admission budget in bytes                      */
-  uint64_t hbm_in_use;   /* bytes held by live jobs                        */
+  uint64_t hbm_in_use;   /* bytes live jobs need                           */
   int32_t live_jobs;
   int32_t device;
   int64_t kernel_launches; /* kernels this context has launched            */
@@ -163,7 +163,11 @@ int32_t oidt_destroy(oidt_ctx *ctx);
 const char *oidt_last_error(oidt_ctx *ctx);
 int32_t oidt_stats_get(oidt_ctx *ctx, oidt_stats *out);
 
-/* Device bytes a job with this descriptor would hold (admission check). */
+/* Device bytes a job with this descriptor needs (admission check).  2D
+ * tile-form jobs run faster with some more (longer blocks, exchange words
+ * between tiles; at most 34 MB and a ring of 128 steps), which they take
+ * where the budget has room and give back when another job needs it; results
+ * do not depend on it. */
 int32_t oidt_job_bytes(const oidt_job_desc *desc, uint64_t *bytes);
 
 /* Allocate device state, copy the descriptor's host arrays (H2D), zero the

@@ -62,7 +62,6 @@ constexpr int kVariantCell = 0, kVariantSweep = 1, kVariantVec = 2, kVariantWave
 constexpr int kVariantTile = 4;  // 2D: tiles advanced in sub-blocks of up to kTileHaloMax steps (tile2d.cuh)
 constexpr int kTileLongBlock = 128;  // steps of a 2D tile-form job's long block at most (a multiple of its ring block)
 constexpr int kTileMaxBlocks = 1024;  // tiles of a cooperative (several sub-block) launch at most
-constexpr long long kStripCoopCells = 148LL * kStripThreads * kStripCells;  // cells of a grid one cooperative strip launch holds at most
 constexpr size_t kTileSmemMax = 227 * 1024;  // shared memory of a tile block at most
 
 // ---------------------------------------------------------------------------
@@ -373,11 +372,10 @@ struct JobPlan {
   bool mat;
   size_t off_wave;                // ordered form: E-block counts per plane (after 8 spare bytes)
   size_t off_tile;                // 2D tile form: sub-blocks completed per tile [kTileMaxBlocks] ...
-  bool strip;                     // ... the strip kernel (float32 fast; else one cell a thread) ...
-  size_t off_xch, xch_words;      // ... and exchange words (0: none)
+  bool strip;                     // ... the strip kernel (float32 fast; else one cell a thread)
   size_t off_pow;                 // port power [nf] complex float64
   long long N, plane;
-  int K, KL, esz, nzp, nbuf, variant, L, nitems;  // K: steps of a ring block; KL: of a long block (K but for the tile form)
+  int K, KL, esz, nzp, nbuf, variant, L, nitems;  // K: steps of a ring block; KL: of a long block (K but for the tile form; Job::xmem)
   int rows;  // 3D per-cell tile rows
   int psi_pitch;  // row length along z of the 3D x- and y-slab psi arrays (nz or nzp)
   int psz;        // row length of the 3D z-slab psi arrays (P, or the vector form's padded rows) ...
@@ -472,6 +470,9 @@ long long vec_blocks_per_plane(const oidt_job_desc *d, int nzp) {
   const VecGeom g = vec_geom_of(d->kb, d->ke, d->num_cpml, d->jb, d->je, nzp, 4);
   return (long long)g.nb_vec + vec_edge_blocks(g, d->jb, d->je, 4);
 }
+
+// The capture ring of K steps.
+size_t ring_bytes(int mode, int K, long long plane, int esz) { return (size_t)K * 2 * nslot_of(mode) * plane * esz; }
 
 int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
   auto bad = [&](const char *m) { if (why) *why = m; return OIDT_ERR_INVALID; };
@@ -591,11 +592,11 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
             L.take(psi_elems(d->mode, fa.second, d->nx, d->ny, d->nz, P, psi_pitch, zr.pitch) * esz);
   pl->off_jsrc = L.take((size_t)d->nt * esz);
   for (int t = 0; t < 4; ++t) pl->off_tw[t] = L.take((size_t)d->nf * d->nt * 8);
-  // Tile form: a ring of KL >= K steps.  An advance of KL steps or more replays blocks of KL, whose launch, set-up
-  // and fold (7 us a block, a fifth of a 32-step block of a 400 x 200 slab) are paid once; multi-job blocks stay K.
-  // Planes of 20000 cells and more keep blocks of K: their steps are far longer, their rings not small.
+  pl->off_ring = L.take(ring_bytes(d->mode, K, plane, esz));
+  // Tile form: long blocks of KL >= K steps.  An advance of KL steps or more replays blocks of KL, whose launch,
+  // set-up and fold (7 us a block, a fifth of a 32-step block of a 400 x 200 slab) are paid once; multi-job blocks
+  // stay K.  Planes of 20000 cells and more keep blocks of K: their steps are far longer, their rings not small.
   const int KL = variant == kVariantTile && K < kTileLongBlock && plane < 20000 ? kTileLongBlock / K * K : K;
-  pl->off_ring = L.take((size_t)KL * 2 * nslot_of(d->mode) * plane * esz);
   pl->off_acc = L.take((size_t)2 * ncomp_of(d->mode) * d->nf * plane * 16);
   pl->off_state = L.take(64);
   pl->off_pow = L.take((size_t)d->nf * 16);
@@ -607,13 +608,7 @@ int plan_job(const oidt_job_desc *d, JobPlan *pl, std::string *why) {
   if (variant == kVariantWave) pl->off_wave = L.take(8 + (size_t)4 * (d->ie - d->ib));
   if (variant == kVariantTile) {
     pl->off_tile = L.take((size_t)4 * kTileMaxBlocks);
-    // exchange words (34 MB at most), for grids a cooperative launch can hold
     pl->strip = d->precision == OIDT_F32 && d->arith == OIDT_ARITH_FAST;
-    const long long most = pl->strip ? kStripCoopCells : 148LL * kTileThreads;
-    pl->xch_words = d->reserved[2] != 0 || N > most || (long long)P * (d->nx + d->ny) > most ? 0
-                    : pl->strip ? 2 * strip2d_xch_buf(d->nx, d->ny, P)
-                                : 2 * tile2d_xch_buf(esz, d->nx, d->ny, P);
-    pl->off_xch = L.take(8 * pl->xch_words);
   }
   if (d->probe[0] == 1) {
     pl->probe_bytes = (size_t)4 * d->nt * d->nx * esz;
@@ -667,6 +662,14 @@ struct Job {
   bool tile_coop = false;               // ... a ring block is one cooperative launch of sub-blocks
   size_t tile_smem = 0;                 // ... shared memory of a block
   StripArgs strip{};                    // ... the strip kernel's split (in place of `tile`)
+  // 2D tile form: memory the job is faster with and can do without -- a ring for long blocks (KL > pl.K), then the
+  // exchange words of cooperative launches (34 MB at most).  Not part of what a job needs (oidt_job_bytes): taken
+  // where the budget has room, given back when a new job needs the room (drop_extra); the job then goes on in
+  // blocks of pl.K steps, a launch per sub-block, with the same results.
+  unsigned char *xmem = nullptr;
+  size_t xbytes = 0, xch_off = 0, xch_words = 0;
+  int KL = 0;                           // steps of the job's long blocks (pl.K: none)
+  std::vector<cudaGraphExec_t> old;     // graphs that may be in flight still, of launches before drop_extra
 };
 
 constexpr int kAuxStreams = 64;  // a served request is two jobs; the mix keeps ~40 active
@@ -680,7 +683,7 @@ struct oidt_ctx {
   cudaStream_t readout = nullptr; // port-power reductions (never queued behind compute)
   cudaStream_t aux[kAuxStreams] = {};  // branches of multi-job blocks
   cudaEvent_t fork = nullptr, join[kAuxStreams] = {};
-  uint64_t budget = 0, in_use = 0;
+  uint64_t budget = 0, in_use = 0, extra_use = 0;  // extra_use: of Job::xmem
   std::map<uint64_t, Job *> jobs;
   uint64_t next_id = 1;
   std::mutex mu;
@@ -809,8 +812,8 @@ template <typename T> void fill_params(Job *J) {
     for (int a = 0; a < 3; ++a) { p.slo[a] = d.src_lo[a]; p.shi[a] = d.src_hi[a]; }
     if (d.mode != OIDT_MODE_YEE3D) { p.slo[2] = 0; p.shi[2] = 1; }
     p.jsrc = reinterpret_cast<const T *>(m + pl.off_jsrc);
-    p.ring = reinterpret_cast<T *>(m + pl.off_ring);
-    p.ring_K = pl.KL;
+    p.ring = reinterpret_cast<T *>(J->KL > pl.K ? J->xmem : m + pl.off_ring);
+    p.ring_K = J->KL;
     p.nslot = nslot_of(d.mode);
     p.plane = pl.plane;
     p.port_pos[0] = d.port_pos[0];
@@ -832,7 +835,7 @@ template <typename T> void fill_params(Job *J) {
   memset(&fp, 0, sizeof fp);
   fp.mode = d.mode; fp.nx = d.nx; fp.ny = d.ny; fp.nf = d.nf; fp.nt = d.nt;
   fp.nslot = nslot_of(d.mode); fp.ncomp = ncomp_of(d.mode); fp.plane = pl.plane;
-  fp.ring = reinterpret_cast<T *>(m + pl.off_ring);
+  fp.ring = reinterpret_cast<T *>(J->KL > pl.K ? J->xmem : m + pl.off_ring);
   fp.acc = reinterpret_cast<double2 *>(m + pl.off_acc);
   for (int t = 0; t < 4; ++t) fp.tw[t] = reinterpret_cast<const double *>(m + pl.off_tw[t]);
   fp.wlo0 = d.win_lo[0]; fp.whi0 = d.win_hi[0]; fp.wlo1 = d.win_lo[1]; fp.whi1 = d.win_hi[1];
@@ -913,6 +916,7 @@ template <typename T> int upload(oidt_ctx *ctx, Job *J, const oidt_job_desc *src
   unsigned char *m = J->mem;
   cudaStream_t st = ctx->upload;
   CU(ctx, cudaMemsetAsync(m, 0, pl.total, st));
+  if (J->xmem) CU(ctx, cudaMemsetAsync(J->xmem, 0, J->xbytes, st));
   std::vector<T> tab;
   std::unique_ptr<uint8_t[]> found;
   // Vector form, dt/eps given as grids: where they hold few materials the E half-step reads one index byte a cell
@@ -1126,8 +1130,8 @@ void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStre
     a.s0 = s0;
     a.cnt = cnt;
     a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
-    a.xch = reinterpret_cast<unsigned long long *>(J->mem + J->pl.off_xch);
-    a.xbuf = (long long)J->pl.xch_words / 2;
+    a.xch = reinterpret_cast<unsigned long long *>(J->xmem + J->xch_off);
+    a.xbuf = (long long)J->xch_words / 2;
     tile_launch_as(p.mode == OIDT_MODE_TM2 ? strip_kernel<OIDT_MODE_TM2>(a.cells) : strip_kernel<OIDT_MODE_TE2>(a.cells),
                    cnt > a.halo, pdl, J->tile_blocks, a.threads, J->tile_smem, st, p, a);
   } else {
@@ -1137,8 +1141,8 @@ void tile_launch(bool pdl, Job *J, const Params<T> &p, int s0, int cnt, cudaStre
     a.s0 = s0;
     a.cnt = cnt;
     a.epoch = reinterpret_cast<int *>(J->mem + J->pl.off_tile);
-    a.xch = reinterpret_cast<unsigned long long *>(J->mem + J->pl.off_xch);
-    a.xbuf = (long long)J->pl.xch_words / 2;
+    a.xch = reinterpret_cast<unsigned long long *>(J->xmem + J->xch_off);
+    a.xbuf = (long long)J->xch_words / 2;
     tile_launch_as(kern, cnt > a.halo, pdl, J->tile_blocks, kTileThreads, J->tile_smem, st, p, a);
   }
 }
@@ -1258,7 +1262,7 @@ template <typename T, bool EXACT> void launch_steps(oidt_ctx *ctx, Job *J, int c
 // enqueues nothing, so st may hold work of other jobs.
 // lng: the job's long block (KL steps) instead.
 template <typename T, bool EXACT> int job_graph(oidt_ctx *ctx, Job *J, int par, cudaStream_t st, bool lng = false) {
-  const int k = lng ? 2 + par : par, K = lng ? J->pl.KL : J->pl.K;
+  const int k = lng ? 2 + par : par, K = lng ? J->KL : J->pl.K;
   if (J->graph[k]) return OIDT_OK;
   cudaGraph_t g;
   const long long before = ctx->launches;
@@ -1280,8 +1284,8 @@ template <typename T, bool EXACT> int advance_t(oidt_ctx *ctx, Job *J, int nstep
   const int K = J->pl.K;
   int left = nsteps;
   while (left > 0) {
-    const bool lng = left >= J->pl.KL && J->pl.KL > K;
-    const int cnt = lng ? J->pl.KL : std::min(K, left);
+    const bool lng = left >= J->KL && J->KL > K;
+    const int cnt = lng ? J->KL : std::min(K, left);
     const int par = J->parity;
     if (cnt >= K && J->d.reserved[1] == 0) {
       int rc = job_graph<T, EXACT>(ctx, J, par, st, lng);
@@ -1499,7 +1503,9 @@ template <typename T, bool EXACT> int profile_t(oidt_ctx *ctx, Job *J, int nstep
 void destroy_job(oidt_ctx *ctx, Job *J) {
   for (cudaGraphExec_t g : J->graph)
     if (g) cudaGraphExecDestroy(g);
+  for (cudaGraphExec_t g : J->old) cudaGraphExecDestroy(g);
   cudaFreeAsync(J->mem, ctx->stream);  // stream-ordered: no device-wide synchronisation
+  if (J->xmem) cudaFreeAsync(J->xmem, ctx->stream);
   cudaEventDestroy(J->ready);
   cudaEventDestroy(J->done);
   delete J;
@@ -1614,7 +1620,7 @@ void strip_plan(Job *J, int sms, bool coop_ok) {
     const long long tiles = (long long)gi * gj;
     const int hi = std::min(nx, ti + 2 * h), hj = std::min(ny, tj + 2 * h);
     const int thr = (int)align_up((size_t)((hi + C - 1) / C) * hj, 32), most = C == 1 ? 2 * kStripThreads : kStripThreads;
-    const size_t smem = strip2d_smem(hi, hj, C, J->pl.KL);
+    const size_t smem = strip2d_smem(hi, hj, C, J->KL);
     if (thr > most || smem > kTileSmemMax || tiles > 0x7fffffff) return;
     const double warps = thr / 32.0, held = thr * C / 2048.0;
     double t;
@@ -1661,6 +1667,70 @@ void strip_plan(Job *J, int sms, bool coop_ok) {
           --ti;
         }
     }
+}
+
+// The split, block length and extra memory of a tile-form job: with extra
+// memory, long blocks and cooperative launches where the grid fits them;
+// without, blocks of pl.K steps, a launch per sub-block.  False: no tiling.
+bool tile_setup(const oidt_ctx *ctx, Job *J, bool extra) {
+  const oidt_job_desc &d = J->d;
+  const JobPlan &pl = J->pl;
+  const bool coop_ok = extra && ctx->coop && d.reserved[2] == 0;
+  J->KL = extra ? pl.KL : pl.K;
+  J->tile_blocks = 0;
+  J->tile_coop = false;
+  if (pl.strip) {
+    strip_plan(J, ctx->sms, coop_ok && pl.N <= (long long)ctx->sms * kStripThreads * kStripCells);
+  } else {
+    tile_plan(J, ctx->sms);
+    J->tile_smem = tile2d_smem(pl.esz, d.num_cpml, J->tile.ti + 2 * J->tile.halo, J->tile.tj + 2 * J->tile.halo);
+    // a ring block in one launch where every tile is resident at once and a tile's
+    // halo reaches its 8 neighbours only
+    J->tile_coop = coop_ok && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
+                   J->tile.halo <= std::min(J->tile.ti, J->tile.tj) && pl.K > J->tile.halo;
+  }
+  J->xch_words = !J->tile_coop ? 0
+                 : pl.strip    ? 2 * strip2d_xch_buf(d.nx, d.ny, d.num_cpml)
+                               : 2 * tile2d_xch_buf(pl.esz, d.nx, d.ny, d.num_cpml);
+  J->xch_off = J->KL > pl.K ? align_up(ring_bytes(d.mode, J->KL, pl.plane, pl.esz), 256) : 0;
+  J->xbytes = align_up(J->xch_off + 8 * J->xch_words, 256);
+  return J->tile_blocks > 0;
+}
+
+// Gives back a job's extra memory, in the order of the compute stream: what
+// the job has enqueued runs as it was launched, what follows does without.
+// Every slot of the long ring holds the same values where no update writes
+// (k_ring_fill), so the first pl.K of them are the short ring's.
+int drop_extra(oidt_ctx *ctx, Job *J) {
+  cudaStream_t st = ctx->stream;
+  CU(ctx, cudaStreamWaitEvent(st, J->ready, 0));
+  if (J->KL > J->pl.K)
+    CU(ctx, cudaMemcpyAsync(J->mem + J->pl.off_ring, J->xmem, ring_bytes(J->d.mode, J->pl.K, J->pl.plane, J->pl.esz),
+                            cudaMemcpyDeviceToDevice, st));
+  CU(ctx, cudaFreeAsync(J->xmem, st));
+  ctx->extra_use -= J->xbytes;
+  J->xmem = nullptr;
+  for (cudaGraphExec_t &g : J->graph) {
+    if (g) J->old.push_back(g);
+    g = nullptr;
+  }
+  tile_setup(ctx, J, false);
+  if (J->d.precision == OIDT_F64) fill_params<double>(J);
+  else fill_params<float>(J);
+  CU(ctx, cudaEventRecord(J->done, st));
+  J->busy = true;
+  return OIDT_OK;
+}
+
+// Has live jobs give back extra memory until `bytes` more fit the budget.
+int make_room(oidt_ctx *ctx, uint64_t bytes) {
+  for (auto &kv : ctx->jobs) {
+    if (ctx->in_use + ctx->extra_use + bytes <= ctx->budget) break;
+    if (!kv.second->xmem) continue;
+    int rc = drop_extra(ctx, kv.second);
+    if (rc) return rc;
+  }
+  return OIDT_OK;
 }
 
 }  // namespace
@@ -1790,35 +1860,50 @@ int32_t oidt_job_create(oidt_ctx *ctx, const oidt_job_desc *desc, uint64_t *job)
     return fail(ctx, OIDT_ERR_BUDGET, "job needs %llu bytes; %llu of %llu in use", (unsigned long long)pl.total,
                 (unsigned long long)ctx->in_use, (unsigned long long)ctx->budget);
   CU(ctx, cudaSetDevice(ctx->device));
+  rc = make_room(ctx, pl.total);
+  if (rc) return rc;
   Job *J = new Job();
   J->d = *desc;
   J->pl = pl;
+  J->KL = pl.K;
   if (pl.variant == kVariantTile) {
-    if (pl.strip) {
-      strip_plan(J, ctx->sms, ctx->coop && pl.xch_words > 0);
-    } else {
-      tile_plan(J, ctx->sms);
-      J->tile_smem = tile2d_smem(pl.esz, desc->num_cpml, J->tile.ti + 2 * J->tile.halo, J->tile.tj + 2 * J->tile.halo);
-      // a ring block in one launch where every tile is resident at once and a tile's
-      // halo reaches its 8 neighbours only
-      J->tile_coop = ctx->coop && pl.xch_words > 0 && J->tile_blocks <= std::min(ctx->sms, kTileMaxBlocks) &&
-                     J->tile.halo <= std::min(J->tile.ti, J->tile.tj) && J->pl.K > J->tile.halo;
-    }
-    if (J->tile_blocks == 0) {
+    bool ok = tile_setup(ctx, J, true);
+    if (ok && ctx->in_use + ctx->extra_use + pl.total + J->xbytes > ctx->budget) ok = tile_setup(ctx, J, false);
+    if (!ok) {
       delete J;
       return fail(ctx, OIDT_ERR_INVALID, "tile form: no tiling of this grid");
     }
   }
-  if (cudaMallocAsync(reinterpret_cast<void **>(&J->mem), pl.total, ctx->upload) != cudaSuccess) {
+  auto take = [&](unsigned char **m, size_t bytes) {
+    return cudaMallocAsync(reinterpret_cast<void **>(m), bytes, ctx->upload) == cudaSuccess;
+  };
+  bool got = take(&J->mem, pl.total);
+  if (!got && ctx->extra_use) {  // the device has less room than the budget: extra memory gives way here too
+    cudaGetLastError();
+    for (auto &kv : ctx->jobs)
+      if (kv.second->xmem && (rc = drop_extra(ctx, kv.second))) {
+        delete J;
+        return rc;
+      }
+    cudaStreamSynchronize(ctx->stream);
+    got = take(&J->mem, pl.total);
+  }
+  if (!got) {
     delete J;
     cudaGetLastError();
     return fail(ctx, OIDT_ERR_BUDGET, "device allocation of %llu bytes failed", (unsigned long long)pl.total);
+  }
+  if (J->xbytes && !take(&J->xmem, J->xbytes)) {
+    cudaGetLastError();
+    J->xmem = nullptr;
+    tile_setup(ctx, J, false);
   }
   cudaEventCreateWithFlags(&J->ready, cudaEventDisableTiming);
   cudaEventCreateWithFlags(&J->done, cudaEventDisableTiming);
   rc = desc->precision == OIDT_F64 ? upload<double>(ctx, J, desc) : upload<float>(ctx, J, desc);
   if (rc) {
     cudaFreeAsync(J->mem, ctx->upload);
+    if (J->xmem) cudaFreeAsync(J->xmem, ctx->upload);
     cudaStreamSynchronize(ctx->upload);
     cudaEventDestroy(J->ready);
     cudaEventDestroy(J->done);
@@ -1835,6 +1920,7 @@ int32_t oidt_job_create(oidt_ctx *ctx, const oidt_job_desc *desc, uint64_t *job)
   J->id = ctx->next_id++;
   ctx->jobs[J->id] = J;
   ctx->in_use += pl.total;
+  if (J->xmem) ctx->extra_use += J->xbytes;
   *job = J->id;
   return OIDT_OK;
 }
@@ -2173,7 +2259,7 @@ int32_t oidt_job_write_field(oidt_ctx *ctx, uint64_t job, int32_t field, const v
     rc = copy_grid_h2d(ctx, J, J->mem + J->pl.off_f[b][field], src, ctx->upload);
     if (rc) return rc;
   }
-  const long long n = (long long)J->pl.KL * 2 * nslot_of(J->d.mode) * J->pl.plane;
+  const long long n = (long long)J->KL * 2 * nslot_of(J->d.mode) * J->pl.plane;
   const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 8);
   if (J->d.precision == OIDT_F64)
     k_ring_fill<double><<<blocks, 256, 0, ctx->upload>>>(cells<double>(J)[J->parity]);
@@ -2223,6 +2309,7 @@ int32_t oidt_job_release(oidt_ctx *ctx, uint64_t job) {
   CU(ctx, cudaSetDevice(ctx->device));
   CU(ctx, cudaEventSynchronize(J->done));
   ctx->in_use -= J->pl.total;
+  if (J->xmem) ctx->extra_use -= J->xbytes;
   ctx->jobs.erase(job);
   destroy_job(ctx, J);
   return OIDT_OK;
@@ -2253,8 +2340,8 @@ int32_t oidt_job_reset(oidt_ctx *ctx, uint64_t job) {
     CU(ctx, cudaMemsetAsync(J->mem + pl.off_wave, 0, 8 + (size_t)4 * (J->d.ie - J->d.ib), st));
   if (pl.variant == kVariantTile)  // the tiles' sub-block counters: equal (zero) again
     CU(ctx, cudaMemsetAsync(J->mem + pl.off_tile, 0, (size_t)4 * kTileMaxBlocks, st));
-  if (pl.xch_words)  // ... and the exchange words with them
-    CU(ctx, cudaMemsetAsync(J->mem + pl.off_xch, 0, 8 * pl.xch_words, st));
+  if (J->xmem)  // ... and the exchange words with them, and the long ring
+    CU(ctx, cudaMemsetAsync(J->xmem, 0, J->xbytes, st));
   CU(ctx, cudaEventRecord(J->done, st));
   J->busy = true;
   J->steps_enqueued = 0;
