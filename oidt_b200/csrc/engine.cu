@@ -43,6 +43,7 @@
 
 #include "../../include/oidt.h"
 #include "kernels.cuh"
+#include "material.h"
 #include "sweep3d.cuh"
 #include "vec3d.cuh"
 #include "tile2d.cuh"
@@ -862,54 +863,6 @@ int copy_grid_d2h(oidt_ctx *ctx, Job *J, void *dst, const void *src) {
   return OIDT_OK;
 }
 
-// The material index of dt/eps grids that hold at most 256 different (CBX, CBY,
-// CBZ) triples (bit for bit), as the grids of a structure of a few materials
-// do: idx[cell] and the triples [256][4].  False: more than that.  One pass
-// over the grids; runs of one triple (the guide axis is contiguous) go 32 cells
-// at a time.
-template <typename T> bool find_mat(const T *const (&cb)[3], size_t n, uint8_t *idx, std::vector<T> &tab) {
-  using U = std::conditional_t<sizeof(T) == 4, uint32_t, uint64_t>;
-  const U *const x = reinterpret_cast<const U *>(cb[0]), *const y = reinterpret_cast<const U *>(cb[1]),
-                *const z = reinterpret_cast<const U *>(cb[2]);
-  constexpr int kSlots = 1024, kRun = 32;
-  std::vector<int> slot(kSlots, -1);  // open addressing, a quarter full at most
-  U key[256][3];
-  int count = 0, cur = 0;
-  tab.assign((size_t)256 * 4, T(0));
-  U a = 0, b = 0, c = 0;
-  for (size_t q = 0; q < n;) {
-    if (count && q + kRun <= n) {
-      U diff = 0;
-      for (int m = 0; m < kRun; ++m) diff |= (x[q + m] ^ a) | (y[q + m] ^ b) | (z[q + m] ^ c);
-      if (!diff) {
-        std::memset(idx + q, cur, kRun);
-        q += kRun;
-        continue;
-      }
-    }
-    for (const size_t e = std::min(n, q + kRun); q < e; ++q) {
-      if (!count || x[q] != a || y[q] != b || z[q] != c) {
-        a = x[q], b = y[q], c = z[q];
-        uint64_t hash = ((uint64_t)a * 0x9E3779B97F4A7C15ull ^ (uint64_t)b) * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)c;
-        hash = (hash * 0x9E3779B97F4A7C15ull) >> 54;
-        for (;; hash = (hash + 1) % kSlots) {
-          if (slot[hash] < 0) {
-            if (count == 256) return false;
-            slot[hash] = cur = count++;
-            key[cur][0] = a, key[cur][1] = b, key[cur][2] = c;
-            for (int k = 0; k < 3; ++k) tab[(size_t)cur * 4 + k] = cb[k][q];
-            break;
-          }
-          cur = slot[hash];
-          if (key[cur][0] == a && key[cur][1] == b && key[cur][2] == c) break;
-        }
-      }
-      idx[q] = (uint8_t)cur;
-    }
-  }
-  return true;
-}
-
 template <typename T> int upload(oidt_ctx *ctx, Job *J, const oidt_job_desc *src) {
   const oidt_job_desc &d = *src;
   const JobPlan &pl = J->pl;
@@ -926,7 +879,7 @@ template <typename T> int upload(oidt_ctx *ctx, Job *J, const oidt_job_desc *src
   if (!pl.mat && pl.variant == kVariantVec && found_tab(pl) + 256 * 4 * sizeof(T) <= (size_t)pl.N * sizeof(T)) {
     found.reset(new (std::nothrow) uint8_t[cells_n]);
     const T *const cb[3] = {static_cast<const T *>(d.cb[0]), static_cast<const T *>(d.cb[1]), static_cast<const T *>(d.cb[2])};
-    J->found_mat = found && find_mat<T>(cb, cells_n, found.get(), tab);
+    J->found_mat = found && find_mat<T>(cb, d.nx, (size_t)d.ny * d.nz, found.get(), tab) == cells_n;
   }
   if (J->found_mat) {
     const size_t row = d.nz, rows = (size_t)d.nx * d.ny;
