@@ -925,7 +925,7 @@ template <typename T> int upload(oidt_ctx *ctx, Job *J, const oidt_job_desc *src
   for (int t = 0; t < 4; ++t)
     CU(ctx, cudaMemcpyAsync(m + pl.off_tw[t], tw[t], (size_t)d.nf * d.nt * 8, cudaMemcpyHostToDevice, st));
   fill_params<T>(J);
-  if (pl.mat) {  // dt/eps grids from the index, for the forms and cells that read them
+  if (pl.mat) {  // dt/eps grids from the index, for the forms that read them (the vector and the ordered form do not)
     const Params<T> &p = cells<T>(J)[0];
     const long long n = (long long)d.nx * d.ny * pl.nzp;
     const unsigned blocks = (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16);

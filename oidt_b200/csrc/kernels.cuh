@@ -173,9 +173,6 @@ __device__ __forceinline__ int ld_acquire(const int *p) {
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release(int *p, int v) {
-  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 // ---------------------------------------------------------------------------
 // Job parameters (device-resident copy for batched launches).
@@ -597,7 +594,7 @@ __device__ __forceinline__ void y3_e_masked(const Params<T> &p, int i, int j, in
 
 // H update of one cell (i, j, k) away from the source box (as y3_h_compute;
 // ib, jb >= 1, so every neighbour read stays inside the grid arrays).
-template <typename T, bool EXACT, bool CG = false>
+template <typename T, bool EXACT>
 __device__ __forceinline__ void y3_h_masked(const Params<T> &p, int i, int j, int k, int s) {
   const int P = p.P;
   // nothing is updated outside [ib, ie) x [jb, je); inside, every neighbour
@@ -612,11 +609,11 @@ __device__ __forceinline__ void y3_h_masked(const Params<T> &p, int i, int j, in
   // Hz i (ib,ie) j (jb,je) k [kb,ke)
   const bool ko = k > p.kb && k < p.ke, kc = k >= p.kb && k < p.ke;
   const bool mhx = j > p.jb && ko, mhy = i > p.ib && ko, mhz = i > p.ib && j > p.jb && kc;
-  const T ex0 = ld_e<CG>(ex + o), ey0 = ld_e<CG>(ey + o), ez0 = ld_e<CG>(ez + o);
+  const T ex0 = __ldg(ex + o), ey0 = __ldg(ey + o), ez0 = __ldg(ez + o);
   // (k - 1 is read only where k > kb >= 1)
-  const T dey_z = A::sub(ey0, ko ? ld_e<CG>(ey + (o - 1)) : ey0), dez_y = A::sub(ez0, ld_e<CG>(ez + (o - sy)));
-  const T dez_x = A::sub(ez0, ld_e<CG>(ez - sx + o)), dex_z = A::sub(ex0, ko ? ld_e<CG>(ex + (o - 1)) : ex0);
-  const T dex_y = A::sub(ex0, ld_e<CG>(ex + (o - sy))), dey_x = A::sub(ey0, ld_e<CG>(ey - sx + o));
+  const T dey_z = A::sub(ey0, ko ? __ldg(ey + (o - 1)) : ey0), dez_y = A::sub(ez0, __ldg(ez + (o - sy)));
+  const T dez_x = A::sub(ez0, __ldg(ez - sx + o)), dex_z = A::sub(ex0, ko ? __ldg(ex + (o - 1)) : ex0);
+  const T dex_y = A::sub(ex0, __ldg(ex + (o - sy))), dey_x = A::sub(ey0, __ldg(ey - sx + o));
   const T rkx = p.rkd[3][i], rky = p.rkd[4][j], rkz = p.rkd[5][k];
   const T kx = EXACT ? p.kd[3][i] : T(0), ky = EXACT ? p.kd[4][j] : T(0), kz = EXACT ? p.kd[5][k] : T(0);
   const T db = p.db;
