@@ -43,6 +43,7 @@
 
 #include "../../include/oidt.h"
 #include "kernels.cuh"
+#include "kappa.h"
 #include "material.h"
 #include "sweep3d.cuh"
 #include "vec3d.cuh"
@@ -904,16 +905,14 @@ template <typename T> int upload(oidt_ctx *ctx, Job *J, const oidt_job_desc *src
     }
   }
   const int dims[3] = {d.nx, d.ny, d.nz};
-  std::vector<T> rk;
+  std::vector<T> kp, rk;
   for (int a = 0; a < 6; ++a) {
     if (d.mode != OIDT_MODE_YEE3D && (a == 2 || a == 5)) continue;
-    const int n = dims[a % 3];
-    const T *kd = static_cast<const T *>(d.kdx[a]);
-    CU(ctx, cudaMemcpyAsync(m + pl.off_kd[a], kd, n * sizeof(T), cudaMemcpyHostToDevice, st));
-    rk.resize(n);
-    for (int i = 0; i < n; ++i) rk[i] = (T)1 / kd[i];  // RN(1/kd) in T (EXACT divisions rely on it)
+    const size_t n = align_up(dims[a % 3], 4);
+    kappa_rows<T>(static_cast<const T *>(d.kdx[a]), dims[a % 3], n, kp, rk);
+    CU(ctx, cudaMemcpyAsync(m + pl.off_kd[a], kp.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
     CU(ctx, cudaMemcpyAsync(m + pl.off_rkd[a], rk.data(), n * sizeof(T), cudaMemcpyHostToDevice, st));
-    CU(ctx, cudaStreamSynchronize(st));  // rk is reused
+    CU(ctx, cudaStreamSynchronize(st));  // kp and rk are reused
   }
   const int P = d.num_cpml;
   CU(ctx, cudaMemcpyAsync(m + pl.off_be, d.be, P * sizeof(T), cudaMemcpyHostToDevice, st));
