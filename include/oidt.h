@@ -106,8 +106,9 @@ typedef struct oidt_job_desc {
   int32_t ring_steps; /* steps buffered between DFT folds (0 = default)    */
   /* reserved[0]: launch form.  3D: 0 = per-cell E-half / H-half launches,
    *              1 = plane sweep (one launch per step),
-   *              2 = vector form: the E-half / H-half launches with four
-   *                  cells per thread along z and 16-byte accesses,
+   *              2 = vector form: the E-half / H-half launches with 16
+   *                  bytes of cells (four float32, two float64) per thread
+   *                  along z,
    *              3 = ordered form: the vector form's code in one launch per
    *                  step, E and H half-steps ordered plane by plane.
    *              2D: 0 = per-cell E-half / H-half launches,
@@ -115,7 +116,7 @@ typedef struct oidt_job_desc {
    *                  halo around it through sub-blocks of up to 8 steps in
    *                  shared memory; a ring block is one cooperative launch
    *                  where every tile is resident at once, and so is a
- *                  block of up to 128 steps of a long advance;
+   *                  block of up to 128 steps of a long advance;
    * reserved[1]: 1 = launch every step directly (no CUDA-graph replay);
    * reserved[2]: 3D per-cell form: rows of a block's 32 x rows tile,
    *              2, 4 or 8 (0 = 4); 2D tile form: 1 = one launch per

@@ -1556,7 +1556,7 @@ void tile_plan(Job *J, int sms) {
 // launch per sub-block in waves.  The estimates' constants are fits to steps
 // measured on a B200 (us per step, best of each kind: one cell a thread / four
 // / waves): 300 x 150 0.94 / 1.30 / 1.9, 400 x 200 1.13 / 1.38 / 2.2,
-// 480 x 250 2.44 / 1.48 / 2.8, 613 x 227 - / 1.57 / 2.2, 675 x 141 TE 1.55 /
+// 480 x 250 2.44 / 1.48 / 2.8, 613 x 227 - / 1.57 / 2.2, 675 x 141 1.55 /
 // 1.44 / 1.9, 800 x 300 - / 2.23 / 3.5, 603 x 1601 - / - / 10.9.  Among equal
 // estimates the tile nearest a square wins: 613 x 227 at 4 steps 1.60 with
 // 26 x 38 tiles, 1.71 with 13 x 76, 1.98 with 103 x 10.

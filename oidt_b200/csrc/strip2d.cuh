@@ -40,14 +40,15 @@
 // an L2 store and load a crossing.  Strips of four hold twice the cells of a
 // block and hide the chain; strips of one have the shorter half-step, for
 // grids of which 148 tiles hold a thread's worth a cell (engine.cu,
-// strip_plan).  Measured on a B200 against the one-cell form with its state
-// exchanged through global memory behind counters: 613 x 227 1.57 against
-// 3.30 us per step (that form ran in waves there), 675 x 141 TE 1.43 / 2.6,
-// 400 x 200 1.13 / 1.75, 603 x 1601 10.9 / 21.3.
+// strip_plan).  Measured on a B200 (advances of 2560 steps, folds included)
+// against the one-cell form with its state exchanged through global memory
+// behind counters: 613 x 227 1.57 against 3.46 us per step (that form ran in
+// waves there), 675 x 141 1.46 / 2.99, TE 1.71 / 3.14, 400 x 200 1.13 / 1.81,
+// 603 x 1601 10.9 / 21.7.
 //
 // float64 and EXACT runs stay in tile2d.cuh's one-cell form: with strips their
-// registers spill (float64 fast 2.20 against 2.05 us per step of the
-// 400 x 200 slab, exact 3.57 against 2.87).
+// registers spill (400 x 200, us per step: float64 fast 2.20, EXACT 3.57; the
+// one-cell form 2.05 and 2.87 then, 1.64 and 2.30 now).
 //
 // Per cell the arithmetic is that of kernels.cuh's tm2_e_cell / tm2_h_cell /
 // te2_e_cell / te2_h_cell (the reference's fdtd_funcs.py of FDTD_2D_TM and

@@ -43,7 +43,8 @@ constexpr int kVecThreads = 128;
 // blocks (64 registers) spill more and lose (76.1).
 // FP64 with two cells a thread: 97 x 114 x 187 fast 63.9 us per step with
 // seven / six blocks, 64.9 with six / six, 66.7 with six / five; EXACT 107.3,
-// 103.8, 101.7 (99.4 with v3_src_e out of line).
+// 103.8, 101.7 (79.5 now, with the source terms in SRC instances only and the
+// kappa tables' padding in the quotients' range).
 template <typename T, bool EXACT> constexpr int kVecBlocksPerSM = sizeof(T) == 8 && EXACT ? 5 : 6;   // H half-step
 template <typename T, bool EXACT> constexpr int kVecBlocksPerSME = sizeof(T) == 8 && EXACT ? 6 : 7;  // E half-step
 
@@ -175,8 +176,8 @@ __device__ __forceinline__ void psi_prefetch(const Params<T> &p, int i, int j, i
 // `yin`) and one branch for all of them, so that their chains overlap.
 // Measured on a B200, 97 x 114 x 187 float64 EXACT: 144 us per step with a
 // test and a branch a quotient, 117 with one a cell, 120 with one a group of
-// four cells, 102 with one a group of two (and six / five blocks an SM; 99 now);
-// float32 EXACT 88, 84 and 64.
+// four cells, 102 with one a group of two (and six / five blocks an SM; 79.5 now,
+// see kVecBlocksPerSM and kappa.h); float32 EXACT 88, 84 and 64.
 template <typename T, bool EXACT> __device__ __forceinline__ bool yin3(T y) {
   if constexpr (EXACT) return Ar<T, EXACT>::yin(y);
   else return true;

@@ -117,14 +117,15 @@ def to_desc(spec: SimSpec, arith: str = "fast", precision=None, ring_steps: int 
     ``keepalive`` must outlive the ``oidt_job_create`` call.
 
     ``variant``: 'auto' (default) picks 'vec' in 3D and 'tile' in 2D.
-    3D: 'vec' -- the E-half / H-half launches with four cells per thread
-    along z and 16-byte accesses; 'wave' -- the same code in one launch per
-    step, E and H half-steps ordered plane by plane; 'cell' -- the
+    3D: 'vec' -- the E-half / H-half launches with 16 bytes of cells (four
+    float32, two float64) per thread along z; 'wave' -- the same code (four
+    cells) in one launch per step, E and H half-steps ordered plane by
+    plane; 'cell' -- the
     half-steps with one cell per thread; 'sweep' -- one plane-sweep launch
     per step (E and H fused, TMA-staged tiles).  2D: 'cell' -- the E-half /
     H-half launches with one cell per thread; 'tile' -- each block advances
-    a tile of the grid (and a halo around it) in shared memory through
-    sub-blocks of up to 8 steps.  ``tile_steps`` (2D tile form): steps per
+    a tile of the grid (and a halo around it) in registers and shared memory
+    through sub-blocks of up to 8 steps.  ``tile_steps`` (2D tile form): steps per
     sub-block, 1 to 8 (0 = the engine's estimate); ``tile_coop``: a ring
     block in one cooperative launch where every tile fits on the device at
     once (default), else one launch per sub-block.  ``graphs=False``

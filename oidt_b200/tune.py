@@ -4,8 +4,9 @@ results unchanged and keep the fastest.
 The choices are ``Engine.submit`` keywords:
 
 * ``variant`` -- 'cell', the per-cell E-half / H-half launches; 'vec', the
-  same half-steps with four cells per thread along z and 16-byte accesses;
-  or 'sweep', one fused plane-sweep launch per step (TMA-staged tiles);
+  same half-steps with 16 bytes of cells (four float32, two float64) per
+  thread along z; 'wave', the vector code in one launch per step; or
+  'sweep', one fused plane-sweep launch per step (TMA-staged tiles);
 * ``rows`` -- per-cell form: a block is a tile of 32 cells along z (the guide
   axis, contiguous) by ``rows`` rows along y, rows 2, 4 or 8;
 * ``march_depth`` -- plane sweep: x-planes per work item (0 = the engine's
